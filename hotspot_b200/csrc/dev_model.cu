@@ -237,23 +237,21 @@ int upload_layers(hsb_dev_model *m) {
 
 static void free_model(hsb_dev_model *m) {
   if (!m) return;
+  if (m->exact && m->exact_free) m->exact_free(m->exact);
   if (m->fast && m->fast_free) m->fast_free(m->fast);
   if (m->mg && m->mg_free) m->mg_free(m->mg);
   if (m->krylov && m->krylov_free) m->krylov_free(m->krylov);
-  double **bufs[] = {&m->y, &m->ys, &m->pgrid, &m->k1, &m->k2, &m->k3, &m->ytemp, &m->t1, &m->t2,
-                     &m->rN, &m->rS, &m->rW, &m->rE, &m->rA, &m->rB, &m->cap, &m->aN, &m->aS,
+  double **bufs[] = {&m->y, &m->ys, &m->pgrid, &m->ytemp, &m->rN, &m->rS, &m->rW, &m->rE, &m->rA, &m->rB, &m->cap, &m->aN, &m->aS,
                      &m->aW, &m->aE, &m->aO, &m->qin, &m->b2g_occ, &m->b2g_area, &m->blk_in,
                      &m->blk_out, &m->gs_delta, &m->trace_buf};
   for (double **b : bufs)
     if (*b) cudaFree(*b);
-  if (m->errbits) cudaFree(m->errbits);
   if (m->pk) cudaFree(m->pk);
   if (m->L0) cudaFree(m->L0);
   if (m->b2g_ptr) cudaFree(m->b2g_ptr);
   if (m->b2g_blk) cudaFree(m->b2g_blk);
   if (m->g2b) cudaFree(m->g2b);
   if (m->gs_status) cudaFree(m->gs_status);
-  if (m->h_err) cudaFreeHost(m->h_err);
   if (m->h_blk) cudaFreeHost(m->h_blk);
   for (auto &g : m->ivg)
     if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -319,11 +317,9 @@ int hsb_dev_create(hsb_dev_model **out, const hsb_grid_desc *d) {
   {
     const size_t vb = sizeof(double) * (size_t)m->vlen;
     ALLOC(m->y, vb); ALLOC(m->ys, vb); ALLOC(m->pgrid, vb);
-    ALLOC(m->k1, vb); ALLOC(m->k2, vb); ALLOC(m->k3, vb);
-    ALLOC(m->ytemp, vb); ALLOC(m->t1, vb); ALLOC(m->t2, vb);
+    ALLOC(m->ytemp, vb);
     cudaMemsetAsync(m->y, 0, vb, m->stream);
     cudaMemsetAsync(m->ys, 0, vb, m->stream);
-    ALLOC(m->errbits, sizeof(unsigned long long));
     ALLOC(m->pk, sizeof(package_RC_t));
     ALLOC(m->L0, sizeof(LayerCoef) * HSB_MAX_LAYERS);
     const size_t bb = sizeof(double) * (size_t)(d->total_n_blocks + d->n_extra);
@@ -331,8 +327,7 @@ int hsb_dev_create(hsb_dev_model **out, const hsb_grid_desc *d) {
     ALLOC(m->blk_out, bb);
     ALLOC(m->gs_status, 4 * sizeof(int));
     ALLOC(m->gs_delta, 4 * sizeof(double));
-    if (cudaMallocHost((void **)&m->h_err, sizeof(double) * 4) != cudaSuccess ||
-        cudaMallocHost((void **)&m->h_gs, 4 * sizeof(int)) != cudaSuccess ||
+    if (cudaMallocHost((void **)&m->h_gs, 4 * sizeof(int)) != cudaSuccess ||
         cudaMallocHost((void **)&m->h_gsd, 4 * sizeof(double)) != cudaSuccess ||
         cudaMallocHost((void **)&m->h_blk, 3 * bb) != cudaSuccess) {
       rc = set_error(HSB_E_NOMEM, "cudaMallocHost failed");

@@ -73,9 +73,7 @@ struct hsb_dev_model {
   double *y;          // transient state (last_trans)
   double *ys;         // steady state (last_steady)
   double *pgrid;      // grid power
-  double *k1, *k2, *k3, *ytemp, *t1, *t2;
-  unsigned long long *errbits;   // device max-norm accumulator
-  double *h_err;                 // pinned host mirror
+  double *ytemp;      // candidate state of the exact replay
   package_RC_t *pk;   // device package R/C
   hsb::LayerCoef *L0; // finest-level layer table (device)
   hsb::LayerCoef hostL0[HSB_MAX_LAYERS];
@@ -124,6 +122,8 @@ struct hsb_dev_model {
   // 2 the temporally blocked one with FP64 passes
   int fast_passes;
   int tile_oi, tile_oj;          // the blocked kernel's own tile requested for this model (0: automatic)
+  void *exact;                   // the exact replay's work vectors (rk4_exact.cu), on its first interval
+  void (*exact_free)(void *);
   void *fast;
   void (*fast_free)(void *);
   void *mg;
