@@ -241,8 +241,8 @@ static void free_model(hsb_dev_model *m) {
   if (m->fast && m->fast_free) m->fast_free(m->fast);
   if (m->mg && m->mg_free) m->mg_free(m->mg);
   if (m->krylov && m->krylov_free) m->krylov_free(m->krylov);
-  double **bufs[] = {&m->y, &m->ys, &m->pgrid, &m->ytemp, &m->rN, &m->rS, &m->rW, &m->rE, &m->rA, &m->rB, &m->cap, &m->aN, &m->aS,
-                     &m->aW, &m->aE, &m->aO, &m->qin, &m->b2g_occ, &m->b2g_area, &m->blk_in,
+  double **bufs[] = {&m->y, &m->ys, &m->pgrid, &m->ytemp, &m->rN, &m->rS, &m->rW, &m->rE, &m->rA, &m->rB,
+                     &m->cap, &m->aN, &m->aS, &m->aW, &m->aE, &m->aO, &m->qin, &m->b2g_occ, &m->b2g_area, &m->blk_in,
                      &m->blk_out, &m->gs_delta, &m->trace_buf};
   for (double **b : bufs)
     if (*b) cudaFree(*b);
@@ -258,7 +258,6 @@ static void free_model(hsb_dev_model *m) {
   if (m->ev[0]) cudaEventDestroy(m->ev[0]);
   if (m->ev[1]) cudaEventDestroy(m->ev[1]);
   if (m->h_gs) cudaFreeHost(m->h_gs);
-  if (m->h_gsd) cudaFreeHost(m->h_gsd);
   if (m->levels) {
     for (int l = 1; l < m->n_levels; l++) {
       if (m->levels[l].p) cudaFree(m->levels[l].p);
@@ -327,12 +326,13 @@ int hsb_dev_create(hsb_dev_model **out, const hsb_grid_desc *d) {
     ALLOC(m->blk_out, bb);
     ALLOC(m->gs_status, 4 * sizeof(int));
     ALLOC(m->gs_delta, 4 * sizeof(double));
-    if (cudaMallocHost((void **)&m->h_gs, 4 * sizeof(int)) != cudaSuccess ||
-        cudaMallocHost((void **)&m->h_gsd, 4 * sizeof(double)) != cudaSuccess ||
+    if (cudaMallocHost((void **)&m->h_gs, 128 + HSB_REPORT_BYTES) != cudaSuccess ||
         cudaMallocHost((void **)&m->h_blk, 3 * bb) != cudaSuccess) {
       rc = set_error(HSB_E_NOMEM, "cudaMallocHost failed");
       goto fail;
     }
+    m->h_gsd = (double *)((char *)m->h_gs + 64);
+    m->h_rep = (char *)m->h_gs + 128;
   }
   // nested-iteration levels: halve rows and cols until either reaches 1
   // (recursive_multigrid, temperature_grid.c:2733-2797)

@@ -113,6 +113,8 @@ struct hsb_dev_model {
   double *gs_delta;              // device: last sweep's max change
   int *h_gs;                     // pinned host mirror of gs_status
   double *h_gsd;
+#define HSB_REPORT_BYTES 256
+  void *h_rep;                   // pinned: a kernel's report (HSB_REPORT_BYTES, in h_gs's allocation)
 
   // fast-form workspaces (allocated lazily by those solvers); coef_version
   // counts coefficient uploads so derived FP32 tables are rebuilt when stale

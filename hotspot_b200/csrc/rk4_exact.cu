@@ -23,8 +23,8 @@
 //
 // The package nodes' slopes need sums over the edge rows and columns in the
 // reference's sequential order.  One CTA does them: its other warps bring
-// the edges of the next chunk into shared memory as differences while one
-// lane per edge adds up the current one; then one lane per node.
+// the edges of the next chunk into shared memory while one lane per edge adds
+// up the current one; then one lane per node.
 //
 // Step control is the reference's.  Its pow() is the C library's, evaluated
 // on the host; the kernel goes on by itself wherever the result is already
@@ -33,9 +33,13 @@
 // within 1e-9), which is every step of an ordinary interval, and hands the
 // error norm back to the host where it is not.
 //
-// Measured on one B200 against one launch per stage, with a host round trip
-// per attempt (and the package block's lanes reading their edges from global
-// memory one dependent load after another): see the table in rk4_exact_run.
+// Measured on one B200, an interval of four steps through compute_temp, one
+// launch per stage with a host round trip per attempt against this kernel:
+// 64x64x4 632 -> 175 us, 256x256x6 1440 -> 378 us, a 128x128x4 microchannel
+// stack (14 attempts, 8 of them decided on the host) 2260 -> 770 us.  A grid
+// barrier is 2.1 thousand cycles of a pass; at 64x64x4 the package CTA's pass
+// is 4.3 to 6 thousand (an FP64 add is 18 cycles, so a 64-cell edge 1.2), at
+// 256x256x6 the cells' is 13.5 for one stage input and 19 for two.
 #include <cmath>
 #include <cstring>
 
@@ -43,7 +47,10 @@
 
 namespace hsb {
 
-#define XT 512              // threads per CTA: a tile of cells of one layer
+// threads per CTA at most, a tile of cells of one layer: 128 registers hold
+// what two stage inputs of a cell read; at 1024 threads (64 registers) the
+// spills cost more than the warps give (256x256x6: 479 us against 366)
+#define XTMAX 512
 #define XCHUNK 128          // edge cells per chunk of the package CTA
 #define XNX (HSB_EXTRA + HSB_EXTRA_SEC)
 #define XBAR_LIMIT (1 << 22)   // polls before a grid barrier is given up
@@ -56,15 +63,6 @@ namespace hsb {
 #define DELTA 1.0e-6
 #define HMIN(x, y) (((x) < (y)) ? (x) : (y))
 
-// the package node equations of pack_slope (temperature_grid.c:2857-3093),
-// one row per node: dv = (edge sum / edgeR + (t0 + t1 + t2)) / C, with
-// t_q = (x_nb - x) / R; every resistance is the double the reference divides by
-struct PackX {
-  double edgeR[XNX], C[XNX], R[XNX][3];
-  int eidx[XNX];              // edge sum (edge_desc order), -1 none
-  int nb[XNX][3];             // node, -1 ambient; terms [0, nt)
-  int nt[XNX];
-};
 
 struct XCtl {                 // the kernel's report
   double t, h, max;
@@ -75,11 +73,19 @@ struct XCtl {                 // the kernel's report
 };
 enum { X_DONE = 0, X_POW = 1 };
 
+// per-cell coefficients: reciprocals of A.rN, rS, rE, rW, rA, rB and cap, one array after another
+struct XField {
+  const double *z;
+};
+
+struct PackX;
 struct XArgs {
   StencilArgs A;
+  XField F;
   const PackX *px;
   int el[5];                  // layers of the edge groups in edge_desc order
   int txl;                    // log2 of the tile width
+  int cwl;                    // log2 of the package CTA's chunk width
   int tiles, ntj, nti;
   double *Y[2], *k[3], *X[4], *acc[2], *t1;
   const double *p;
@@ -96,10 +102,12 @@ struct XWork {
   double *v[10];
   unsigned *bar;
   unsigned long long *err;
-  XCtl *ctl, *h_ctl;
+  XCtl *ctl;
   PackX *px;
+  double *z;                  // reciprocals of the per-cell coefficients (field models)
   int px_version;
-  int grid[4];                // co-resident CTAs per kernel variant
+  int nsm;
+  bool ready[4];              // per kernel variant: shared memory limit raised
 };
 
 // grid barrier: one arrival per CTA on a counter that only grows
@@ -132,6 +140,70 @@ struct XForm {
   __device__ __forceinline__ double operator()(long long c) const { return y[c] + a * k[c]; }
 };
 
+// x / y for a divisor known in advance, correctly rounded: with zh = RN(1/y)
+// and zl = RN(1/y - zh), q1 = RN(zh x + RN(zl x)) is a faithful quotient
+// (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Computers 2004), and one correction with its exact remainder rounds it
+// correctly (Markstein's theorem, IBM J. R&D 1990).  Four multiply-adds in
+// place of a division's reciprocal iteration.  Both proofs need quotients
+// clear of underflow and overflow: `bad` collects results outside 2^-819 ..
+// 2^813 (infinities and NaN included), and the cell is then evaluated with
+// plain divisions.  Zero over anything is exact as it is.
+struct XDiv {
+  double y, zh, zl;
+};
+__device__ __forceinline__ bool xrange_bad(double q, double x) {
+  return ((unsigned)__double2hiint(q) & 0x7fffffffu) - 0x0cc00000u >= 0x66000000u &&
+         ((unsigned)__double2hiint(x) & 0x7fffffffu) != 0u;
+}
+__device__ __forceinline__ double xdiv(double x, const XDiv &d, bool &bad) {
+  const double q1 = __fma_rn(d.zh, x, __dmul_rn(d.zl, x));
+  const double q = __fma_rn(__fma_rn(-d.y, q1, x), d.zh, q1);
+  bad |= xrange_bad(q, x);
+  return q;
+}
+// the same from y and zh alone (per-cell coefficients): the faithful
+// quotient from one more remainder step instead of zl
+__device__ __forceinline__ double xdiv(double x, double y, double zh, bool &bad) {
+  const double q0 = __dmul_rn(x, zh);
+  const double q1 = __fma_rn(__fma_rn(-y, q0, x), zh, q0);
+  const double q = __fma_rn(__fma_rn(-y, q1, x), zh, q1);
+  bad |= xrange_bad(q, x);
+  return q;
+}
+__host__ __device__ inline XDiv xdivisor(double y) {
+  XDiv d;
+  d.y = y;
+  d.zh = 1.0 / y;
+  d.zl = fma(-y, d.zh, 1.0) / y;
+  return d;
+}
+__device__ __forceinline__ double xdiv6(double x) {
+  const XDiv six = {6.0, 1.0 / 6.0, 0x1p-56 / 6.0 * 4.0};   // 1/6 - RN(1/6) = 2^-54 / 6
+  bool bad = false;
+  const double q = xdiv(x, six, bad);
+  return bad ? x / 6.0 : q;
+}
+
+// the package node equations of pack_slope (temperature_grid.c:2857-3093),
+// one row per node: dv = (edge sum / edgeR + (t0 + t1 + t2)) / C, with
+// t_q = (x_nb - x) / R; every resistance is the double the reference divides
+// by.  A node with fewer terms has itself as the neighbour of the others,
+// which then add zero.
+struct PackX {
+  XDiv edgeR[XNX], C[XNX], R[XNX][3];
+  int eidx[XNX];              // edge sum (edge_desc order), -1 none
+  int nb[XNX][3];             // node, -1 ambient
+  int nt[XNX];
+};
+
+// a layer's divisors
+struct LayerX {
+  XDiv ns, ew, up, dn, edgeNS, edgeEW, amb, cap;
+  int kind, base;             // package nodes W, E, N, S of the layer's edges: base + 0..3
+};
+
 // what a pass does with the slopes of its (up to two) stage inputs at cell or
 // node c; the operation order is that of rk4_core (RCutil.c:469-527)
 enum { XP_K1, XP_1, XP_2, XP_3, XP_4, XP_4S, XP_5, XP_6, XP_7 };
@@ -142,159 +214,405 @@ struct XRole {
   double h, hb;               // full and half step
 };
 
+// the cell's own operands, loaded before its slopes are formed so that they
+// travel together with its neighbours' values
+struct XOwn {
+  double b, c, d;             // stage base; running sums of the one or two cores
+};
 template <int P>
-__device__ __forceinline__ double xepi(const XRole &r, long long c, double ka, double kb) {
+__device__ __forceinline__ XOwn xown(const XRole &r, int c) {
+  XOwn o{0.0, 0.0, 0.0};
+  if (P == XP_1 || P == XP_2 || P == XP_3) o.b = r.y[c];
+  if (P >= XP_4) o.b = r.t1[c];
+  if (P == XP_1) o.c = r.k1[c];
+  if (P == XP_2 || P == XP_3) {
+    o.c = r.acca[c];
+    o.d = r.accb[c];
+  }
+  if (P == XP_5) o.c = r.k1p[c];
+  if (P == XP_6 || P == XP_7) o.c = r.acca[c];
+  if (P == XP_7) o.d = r.yn[c];
+  return o;
+}
+template <int P>
+__device__ __forceinline__ double xepi(const XRole &r, int c, const XOwn &o, double ka, double kb) {
   if (P == XP_K1) {
     r.k1[c] = ka;
   } else if (P == XP_1) {
-    const double y = r.y[c], k1 = r.k1[c];
-    r.acca[c] = k1 + 2 * ka;
-    r.accb[c] = k1 + 2 * kb;
-    r.Xa0[c] = y + r.h / 2.0 * ka;
-    r.Xb0[c] = y + r.hb / 2.0 * kb;
+    r.acca[c] = o.c + 2 * ka;
+    r.accb[c] = o.c + 2 * kb;
+    r.Xa0[c] = o.b + r.h / 2.0 * ka;
+    r.Xb0[c] = o.b + r.hb / 2.0 * kb;
   } else if (P == XP_2) {
-    const double y = r.y[c];
-    r.acca[c] = r.acca[c] + 2 * ka;
-    r.accb[c] = r.accb[c] + 2 * kb;
-    r.Xa1[c] = y + r.h * ka;
-    r.Xb1[c] = y + r.hb * kb;
+    r.acca[c] = o.c + 2 * ka;
+    r.accb[c] = o.d + 2 * kb;
+    r.Xa1[c] = o.b + r.h * ka;
+    r.Xb1[c] = o.b + r.hb * kb;
   } else if (P == XP_3) {
-    const double y = r.y[c];
-    r.yn[c] = y + r.h * (r.acca[c] + ka) / 6.0;
-    r.t1[c] = y + r.hb * (r.accb[c] + kb) / 6.0;
+    r.yn[c] = o.b + xdiv6(r.h * (o.c + ka));
+    r.t1[c] = o.b + xdiv6(r.hb * (o.d + kb));
   } else if (P == XP_4 || P == XP_4S) {
     r.k1p[c] = ka;
     if (P == XP_4S) r.k1n[c] = kb;
-    r.Xa0[c] = r.t1[c] + r.hb / 2.0 * ka;
+    r.Xa0[c] = o.b + r.hb / 2.0 * ka;
   } else if (P == XP_5) {
-    r.acca[c] = r.k1p[c] + 2 * ka;
-    r.Xa1[c] = r.t1[c] + r.hb / 2.0 * ka;
+    r.acca[c] = o.c + 2 * ka;
+    r.Xa1[c] = o.b + r.hb / 2.0 * ka;
   } else if (P == XP_6) {
-    r.acca[c] = r.acca[c] + 2 * ka;
-    r.Xa0[c] = r.t1[c] + r.hb * ka;
+    r.acca[c] = o.c + 2 * ka;
+    r.Xa0[c] = o.b + r.hb * ka;
   } else {
-    const double t2 = r.t1[c] + r.hb * (r.acca[c] + ka) / 6.0;
-    return fabs(r.yn[c] - t2);   // RCutil.c:592
+    const double t2 = o.b + xdiv6(r.hb * (o.c + ka));
+    return fabs(o.d - t2);   // RCutil.c:592
   }
   return 0.0;
 }
 
 struct XShared {
+  XArgs G;                    // the arguments, the layer table replaced by the one below
   LayerCoef L[HSB_MAX_LAYERS];
+  LayerX X[HSB_MAX_LAYERS];
   PackX px;
+  XRole r;                    // the step's buffers (in shared memory to spare registers)
   double xs[2][XNX], es[2][20], dv[2][XNX];
-  double wmax[XT / 32];
+  double wmax[XTMAX / 32];
   int lost;
+  // what the package CTA's functions need of the arguments
+  int ne, nx, nr, nc, cwl;
+  long long ncell, ebase[20]; // ebase: first cell of each edge (edge_desc order)
+  double ambient;
 };
 
-// package nodes of up to two stage inputs (one CTA)
-template <int P, bool TWO, class TA, class TB>
-__device__ __forceinline__ double xpack(const XArgs &G, const StencilArgs &A, XShared &sh, double *buf, const XRole &r,
-                                        const TA &ta, const TB &tb) {
-  const int t = threadIdx.x, ne = A.secondary ? 20 : 8, nv = TWO ? 2 : 1;
-  const int rows = nv * ne;
-  const int len = A.nr > A.nc ? A.nr : A.nc, nch = (len + XCHUNK - 1) / XCHUNK;
-  if (t < A.nx) {
-    sh.xs[0][t] = ta(A.ncell + t);
-    if (TWO) sh.xs[1][t] = tb(A.ncell + t);
+// the cell with plain divisions (out of line: almost never taken)
+template <bool FIELD, bool ADV, class TA>
+__device__ __noinline__ double xslope_plain(const XShared &sh, const TA ta, const double *p, int n, int i, int j) {
+  return slope_cell_exact<FIELD, ADV>(sh.G.A, ta, p, n, i, j, n * sh.G.A.plane + (long long)i * sh.G.A.nc + j);
+}
+
+// What one cell reads, loaded before anything is computed and from clamped
+// indices where a neighbour is missing, so that a cell costs one trip to the
+// L2 and not one per neighbour.
+template <bool FIELD, bool ADV, bool TWO>
+struct XCell {
+  int n, i, j, c;
+  double pw, Ta, Tb, xa[6], xb[TWO ? 6 : 1];   // power, own value, N S E W above below
+  double y[FIELD ? 7 : 1], z[FIELD ? 7 : 1], am[ADV ? 6 : 1];
+  XOwn o;
+};
+
+template <bool FIELD, bool ADV, int P, bool TWO, class TA, class TB>
+__device__ __forceinline__ void xload(const XShared &sh, const TA &ta, const TB &tb, XCell<FIELD, ADV, TWO> &C) {
+  const int nr = sh.nr, nc = sh.nc, nl = sh.G.A.nl, plane = nr * nc, c = C.c, i = C.i, j = C.j, n = C.n;
+  const int at[6] = {i > 0 ? c - nc : c, i < nr - 1 ? c + nc : c, j < nc - 1 ? c + 1 : c, j > 0 ? c - 1 : c,
+                     n > 0 ? c - plane : c, n < nl - 1 ? c + plane : c};
+  C.pw = sh.G.p[c];
+  C.Ta = ta(c);
+  if (TWO) C.Tb = tb(c);
+#pragma unroll
+  for (int f = 0; f < 6; f++) {
+    C.xa[f] = ta(at[f]);
+    if (TWO) C.xb[f] = tb(at[f]);
   }
-  __syncthreads();
-  auto load = [&](int ch, double *b, int t0, int nt) {
-    for (int q = t0; q < rows * XCHUNK; q += nt) {
-      const int row = q / XCHUNK, m = q - row * XCHUNK;
-      const int v = row >= ne ? 1 : 0, e = row - v * ne, which = e & 3, k = ch * XCHUNK + m;
-      const int n = which < 2 ? A.nc : A.nr;
-      if (k >= n) continue;
-      const long long base = (long long)G.el[e >> 2] * A.plane;
-      const long long c = which == 0 ? base + k : which == 1 ? base + (long long)(A.nr - 1) * A.nc + k
-                          : which == 2 ? base + (long long)k * A.nc : base + (long long)k * A.nc + A.nc - 1;
-      // nodes of a group are numbered W, E, N, S; the sums run N, S, W, E
-      const int g = e >> 2;
-      const int node = (g == 0 ? HSB_SINK_C_W : g == 1 ? HSB_SP_W : g == 2 ? HSB_PCB_C_W : g == 3 ? HSB_SOLDER_W
-                        : HSB_SUB_W) + ((which + 2) & 3);
-      b[row * (XCHUNK + 1) + m] = (TWO && v ? tb(c) : ta(c)) - sh.xs[v][node];
+  if constexpr (FIELD) {
+    const StencilArgs &A = sh.G.A;
+    const double *R[7] = {A.rN, A.rS, A.rE, A.rW, A.rA, A.rB, A.cap};
+#pragma unroll
+    for (int f = 0; f < 7; f++) {
+      C.y[f] = R[f][c];
+      C.z[f] = sh.G.F.z[f * A.ncell + c];
     }
-  };
+  }
+  if constexpr (ADV) {
+    const StencilArgs &A = sh.G.A;
+    if ((A.uchan_mask >> n) & 1ull) {
+      const double *R[6] = {A.aN, A.aS, A.aW, A.aE, A.qin, A.aO};
+#pragma unroll
+      for (int f = 0; f < 6; f++) C.am[f] = R[f][c];
+    }
+  }
+  C.o = xown<P>(sh.r, c);
+}
+
+// slopes of one cell for up to two stage inputs: slope_cell_exact's sums in
+// its order, every quotient through xdiv
+template <bool FIELD, bool ADV, bool TWO, class TA, class TB>
+__device__ __forceinline__ void xslope(const XShared &sh, const TA &ta, const TB &tb,
+                                       const XCell<FIELD, ADV, TWO> &C, double &ka, double &kb) {
+  const LayerX &L = sh.X[C.n];
+  const int nr = sh.nr, nc = sh.nc, nl = sh.G.A.nl, i = C.i, j = C.j;
+  const bool has[6] = {i > 0, i < nr - 1, j < nc - 1, j > 0, C.n > 0, C.n < nl - 1};
+  double sa = 0.0, sb = 0.0;
+  bool bad = false;
+#pragma unroll
+  for (int f = 0; f < 6; f++) {
+    if (has[f]) {
+      const XDiv &d = f < 2 ? L.ns : f < 4 ? L.ew : f == 4 ? L.up : L.dn;
+      if constexpr (FIELD) {
+        sa += xdiv(C.xa[f] - C.Ta, C.y[f], C.z[f], bad);
+        if constexpr (TWO) sb += xdiv(C.xb[f] - C.Tb, C.y[f], C.z[f], bad);
+      } else {
+        sa += xdiv(C.xa[f] - C.Ta, d, bad);
+        if constexpr (TWO) sb += xdiv(C.xb[f] - C.Tb, d, bad);
+      }
+    }
+  }
+  if (L.kind != LK_PLAIN) {
+    auto edge = [&](int side, const XDiv &d) {
+      const int node = nl * nr * nc + L.base + side;
+      sa += xdiv(ta(node) - C.Ta, d, bad);
+      if (TWO) sb += xdiv(tb(node) - C.Tb, d, bad);
+    };
+    if (L.kind == LK_SINK || L.kind == LK_PCB) {
+      sa += xdiv(sh.ambient - C.Ta, L.amb, bad);
+      if (TWO) sb += xdiv(sh.ambient - C.Tb, L.amb, bad);
+    }
+    if (i == 0) edge(2, L.edgeNS);
+    if (i == nr - 1) edge(3, L.edgeNS);
+    if (j == nc - 1) edge(1, L.edgeEW);
+    if (j == 0) edge(0, L.edgeEW);
+  }
+  if constexpr (ADV) {
+    if ((sh.G.A.uchan_mask >> C.n) & 1ull) {
+      // N, S, W, E (xa holds N, S, E, W)
+#pragma unroll
+      for (int f = 0; f < 4; f++) {
+        const int g = f == 2 ? 3 : f == 3 ? 2 : f;
+        if (has[g]) {
+          sa += C.am[f] * ((C.xa[g] + C.Ta) / 2.0);
+          if constexpr (TWO) sb += C.am[f] * ((C.xb[g] + C.Tb) / 2.0);
+        }
+      }
+      sa += C.am[4];
+      sa += C.am[5] * C.Ta;
+      if (TWO) {
+        sb += C.am[4];
+        sb += C.am[5] * C.Tb;
+      }
+    }
+  }
+  kb = 0.0;
+  if constexpr (FIELD) {
+    ka = xdiv(C.pw + sa, C.y[6], C.z[6], bad);
+    if (TWO) kb = xdiv(C.pw + sb, C.y[6], C.z[6], bad);
+  } else {
+    ka = xdiv(C.pw + sa, L.cap, bad);
+    if (TWO) kb = xdiv(C.pw + sb, L.cap, bad);
+  }
+  if (bad) {
+    ka = xslope_plain<FIELD, ADV, TA>(sh, ta, sh.G.p, C.n, i, j);
+    if (TWO) kb = xslope_plain<FIELD, ADV, TB>(sh, tb, sh.G.p, C.n, i, j);
+  }
+}
+
+// reciprocals of the per-cell coefficients
+__global__ void xfield_recip(StencilArgs A, double *z) {
+  const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= A.ncell) return;
+  const double *R[7] = {A.rN, A.rS, A.rE, A.rW, A.rA, A.rB, A.cap};
+#pragma unroll
+  for (int f = 0; f < 7; f++) z[f * A.ncell + c] = 1.0 / R[f][c];
+}
+
+// a chunk's edge cells of up to two stage inputs (x, or x + a k with FORM),
+// eight loads in flight per thread
+template <bool FORM>
+__device__ __noinline__ void xpack_load(const XShared &sh, double *b, const double *xa, const double *xb,
+                                        const double *k, double aa, double ab, int rows, int ch, int t0, int nt) {
+  const int ne = sh.ne, cwl = sh.cwl, nr = sh.nr, nc = sh.nc;
+  for (int q0 = t0; q0 < rows << cwl; q0 += 8 * nt) {
+    double u[8], uk[8];
+    int at[8];
+#pragma unroll
+    for (int z = 0; z < 8; z++) {
+      const int q = q0 + z * nt, row = q >> cwl, m = q & ((1 << cwl) - 1), kk = (ch << cwl) + m;
+      const bool v = row >= ne;
+      const int e = v ? row - ne : row, which = e & 3;
+      at[z] = -1;
+      if (row < rows && kk < (which < 2 ? nc : nr)) {
+        const long long c = sh.ebase[e] + (which < 2 ? (long long)kk : (long long)kk * nc);
+        at[z] = v ? -2 - (row * (XCHUNK + 1) + m) : row * (XCHUNK + 1) + m;
+        u[z] = (v ? xb : xa)[c];
+        if (FORM) uk[z] = k[c];
+      }
+    }
+#pragma unroll
+    for (int z = 0; z < 8; z++) {
+      if (at[z] == -1) continue;
+      const int q = at[z] < 0 ? -2 - at[z] : at[z];
+      b[q] = FORM ? u[z] + (at[z] < 0 ? ab : aa) * uk[z] : u[z];
+    }
+  }
+}
+
+// package-node slopes of nv stage inputs into sh.dv (one CTA)
+template <bool FORM>
+__device__ __noinline__ void xpack_slopes(XShared &sh, double *buf, const double *xa, const double *xb,
+                                          const double *k, double aa, double ab, int nv) {
+  const int t = threadIdx.x, w = t >> 5, lane = t & 31;
+  const int ne = sh.ne, cwl = sh.cwl, nx = sh.nx, nr = sh.nr, nc = sh.nc, rows = nv * ne;
+  const int nch = ((nr > nc ? nr : nc) + (1 << cwl) - 1) >> cwl;
+  double xv = 0.0;
+  if (w < nv && lane < nx) {
+    const long long c = sh.ncell + lane;
+    xv = (w ? xb : xa)[c];
+    if (FORM) xv = xv + (w ? ab : aa) * k[c];
+  }
+  xpack_load<FORM>(sh, buf, xa, xb, k, aa, ab, rows, 0, t, blockDim.x);
   const size_t half = (size_t)40 * (XCHUNK + 1);
-  load(0, buf, t, XT);
+  if (w < nv && lane < nx) sh.xs[w][lane] = xv;
   __syncthreads();
   // sequential sums: one lane per edge, one warp per stage input
-  const int w = t >> 5, lane = t & 31;
-  double s = 0.0;
+  double s = 0.0, xn = 0.0;
+  if (w < nv && lane < ne) {
+    // nodes of a group are numbered W, E, N, S; the sums run N, S, W, E
+    const int g = lane >> 2;
+    xn = sh.xs[w][(g == 0 ? HSB_SINK_C_W : g == 1 ? HSB_SP_W : g == 2 ? HSB_PCB_C_W : g == 3 ? HSB_SOLDER_W
+                   : HSB_SUB_W) + ((lane + 2) & 3)];
+  }
   for (int ch = 0; ch < nch; ch++) {
     const double *b = buf + (ch & 1) * half;
     if (w < nv) {
       if (lane < ne) {
-        const int n = ((lane & 3) < 2 ? A.nc : A.nr) - ch * XCHUNK;
+        const int n = ((lane & 3) < 2 ? nc : nr) - (ch << cwl);
         const double *row = b + (w * ne + lane) * (XCHUNK + 1);
-        const int cnt = n < XCHUNK ? n : XCHUNK;
+        const int cnt = n < 1 << cwl ? n : 1 << cwl;
         int m = 0;
-        for (; m + 8 <= cnt; m += 8) {
-          double u[8];
+        if (cnt >= 8) {
+          double u[8], v[8];
 #pragma unroll
-          for (int q = 0; q < 8; q++) u[q] = row[m + q];
+          for (int q = 0; q < 8; q++) u[q] = row[q] - xn;
+          for (; m + 16 <= cnt; m += 8) {   // the next eight are read while these are added
+#pragma unroll
+            for (int q = 0; q < 8; q++) v[q] = row[m + 8 + q] - xn;
+#pragma unroll
+            for (int q = 0; q < 8; q++) s += u[q];
+#pragma unroll
+            for (int q = 0; q < 8; q++) u[q] = v[q];
+          }
 #pragma unroll
           for (int q = 0; q < 8; q++) s += u[q];
+          m += 8;
         }
-        for (; m < cnt; m++) s += row[m];
+        for (; m < cnt; m++) s += row[m] - xn;
       }
     } else if (ch + 1 < nch) {
-      load(ch + 1, buf + ((ch + 1) & 1) * half, t - 32 * nv, XT - 32 * nv);
+      xpack_load<FORM>(sh, buf + ((ch + 1) & 1) * half, xa, xb, k, aa, ab, rows, ch + 1, t - 32 * nv,
+                       blockDim.x - 32 * nv);
     }
-    __syncthreads();
+    if (nch > 1) __syncthreads();
   }
-  if (w < nv && lane < ne) sh.es[w][lane] = s;
-  __syncwarp();
-  if (w < nv && lane < A.nx) {
-    const PackX &p = sh.px;
-    const double x = sh.xs[w][lane];
-    double S = 0.0;
-    for (int q = 0; q < p.nt[lane]; q++) {
-      const int nb = p.nb[lane][q];
-      const double d = ((nb < 0 ? A.ambient : sh.xs[w][nb]) - x) / p.R[lane][q];
-      S = q == 0 ? d : S + d;
+  if (w < nv) {
+    if (lane < ne) sh.es[w][lane] = s;
+    __syncwarp();
+    if (lane < nx) {
+      const PackX &p = sh.px;
+      const double x = sh.xs[w][lane];
+      bool bad = false;
+      double d[3], xd[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const int nb = p.nb[lane][q];
+        xd[q] = (nb < 0 ? sh.ambient : sh.xs[w][nb]) - x;
+        d[q] = xdiv(xd[q], p.R[lane][q], bad);
+      }
+      const int e = p.eidx[lane];
+      const double es = e >= 0 ? sh.es[w][e] : 0.0;
+      const double S = d[0] + d[1] + d[2];
+      double dv = xdiv(e >= 0 ? xdiv(es, p.edgeR[lane], bad) + S : S, p.C[lane], bad);
+      if (bad) {
+        double T = xd[0] / p.R[lane][0].y;
+        for (int q = 1; q < p.nt[lane]; q++) T += xd[q] / p.R[lane][q].y;
+        dv = (e >= 0 ? es / p.edgeR[lane].y + T : T) / p.C[lane].y;
+      }
+      sh.dv[w][lane] = dv;
     }
-    const int e = p.eidx[lane];
-    const double psum = e >= 0 ? sh.es[w][e] / p.edgeR[lane] + S : S;
-    sh.dv[w][lane] = psum / p.C[lane];
   }
   __syncthreads();
-  return t < A.nx ? xepi<P>(r, A.ncell + t, sh.dv[0][t], TWO ? sh.dv[1][t] : 0.0) : 0.0;
+}
+
+__device__ __forceinline__ void xpack(XShared &sh, double *buf, const XVec &a, const XVec &b, int nv) {
+  xpack_slopes<false>(sh, buf, a.x, b.x, nullptr, 0.0, 0.0, nv);
+}
+__device__ __forceinline__ void xpack(XShared &sh, double *buf, const XForm &a, const XForm &b, int nv) {
+  xpack_slopes<true>(sh, buf, a.y, b.y, a.k, a.a, b.a, nv);
 }
 
 // one pass over the grid (all CTAs but the last) and the package nodes (the
 // last CTA)
 template <bool FIELD, bool ADV, int P, bool TWO, class TA, class TB>
-__device__ __forceinline__ double xpass(const XArgs &G, const StencilArgs &A, XShared &sh, double *buf, const XRole &r,
-                                        const TA &ta, const TB &tb) {
-  if (blockIdx.x == gridDim.x - 1) return xpack<P, TWO>(G, A, sh, buf, r, ta, tb);
+__device__ __noinline__ double xpass(XShared &sh, double *buf, const TA ta, const TB tb) {
+  const XRole &r = sh.r;
+  if (blockIdx.x == gridDim.x - 1) {
+    const int t = threadIdx.x, nx = sh.nx, c = (int)sh.ncell + t;
+    XOwn o{0.0, 0.0, 0.0};
+    if (t < nx) o = xown<P>(r, c);
+    xpack(sh, buf, ta, tb, TWO ? 2 : 1);
+    return t < nx ? xepi<P>(r, c, o, sh.dv[0][t], TWO ? sh.dv[1][t] : 0.0) : 0.0;
+  }
   double err = 0.0;
-  const int tx = threadIdx.x & ((1 << G.txl) - 1), ty = threadIdx.x >> G.txl, th = XT >> G.txl;
-  for (int tile = blockIdx.x; tile < G.tiles; tile += gridDim.x - 1) {
-    const int n = tile / (G.ntj * G.nti), q = tile - n * G.ntj * G.nti;
-    const int bi = q / G.ntj, bj = q - bi * G.ntj;
-    const int i = bi * th + ty, j = (bj << G.txl) + tx;
-    if (i >= A.nr || j >= A.nc) continue;
-    const long long c = (long long)n * A.plane + (long long)i * A.nc + j;
-    const double ka = slope_cell_exact<FIELD, ADV>(A, ta, G.p, n, i, j, c);
-    const double kb = TWO ? slope_cell_exact<FIELD, ADV>(A, tb, G.p, n, i, j, c) : 0.0;
-    err = fmax(err, xepi<P>(r, c, ka, kb));
+  const int txl = sh.G.txl, ntj = sh.G.ntj, nti = sh.G.nti, tiles = sh.G.tiles, nr = sh.nr, nc = sh.nc;
+  const int tx = threadIdx.x & ((1 << txl) - 1), ty = threadIdx.x >> txl, th = blockDim.x >> txl;
+  // a tile's cell of this thread; false outside the grid
+  auto cell = [&](int tile, XCell<FIELD, ADV, TWO> &C) {
+    const int row = tile / ntj;
+    C.n = row / nti;
+    C.i = (row - C.n * nti) * th + ty;
+    C.j = ((tile - row * ntj) << txl) + tx;
+    const bool in = C.i < nr && C.j < nc;
+    C.c = (C.n * nr + C.i) * nc + C.j;   // fewer than 2^31 cells: checked by the host
+    return in;
+  };
+  for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x - 1) {
+    XCell<FIELD, ADV, TWO> C;
+    if (!cell(tile, C)) continue;
+    xload<FIELD, ADV, P, TWO>(sh, ta, tb, C);
+    double ka, kb;
+    xslope<FIELD, ADV, TWO>(sh, ta, tb, C, ka, kb);
+    err = fmax(err, xepi<P>(r, C.c, C.o, ka, kb));
   }
   return err;
 }
 
 template <bool FIELD, bool ADV>
-__global__ void __launch_bounds__(XT, 1) rk4_exact_kernel(const __grid_constant__ XArgs G) {
+__global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_constant__ XArgs G) {
   extern __shared__ double xbuf[];
   __shared__ XShared sh;
   const int tid = threadIdx.x;
-  for (int q = tid; q < G.A.nl * (int)(sizeof(LayerCoef) / 8); q += XT) ((double *)sh.L)[q] = ((const double *)G.A.L)[q];
+  const int nt = blockDim.x;
+  for (int q = tid; q < G.A.nl * (int)(sizeof(LayerCoef) / 8); q += nt) ((double *)sh.L)[q] = ((const double *)G.A.L)[q];
   if (blockIdx.x == gridDim.x - 1)
-    for (int q = tid; q < (int)(sizeof(PackX) / 4); q += XT) ((int *)&sh.px)[q] = ((const int *)G.px)[q];
-  if (tid == 0) sh.lost = 0;
+    for (int q = tid; q < (int)(sizeof(PackX) / 4); q += nt) ((int *)&sh.px)[q] = ((const int *)G.px)[q];
+  if (tid == 0) {
+    sh.lost = 0;
+    sh.G = G;
+    sh.G.A.L = sh.L;
+    sh.ne = G.A.secondary ? 20 : 8;
+    sh.nx = G.A.nx; sh.nr = G.A.nr; sh.nc = G.A.nc; sh.cwl = G.cwl;
+    sh.ncell = G.A.ncell;
+    sh.ambient = G.A.ambient;
+  }
+  if (tid < 20) {
+    const int which = tid & 3;
+    sh.ebase[tid] = (long long)G.el[tid >> 2] * G.A.plane +
+                    (which == 1 ? (long long)(G.A.nr - 1) * G.A.nc : which == 3 ? G.A.nc - 1 : 0);
+  }
   __syncthreads();
-  StencilArgs A = G.A;
-  A.L = sh.L;
+  for (int n = tid; n < G.A.nl; n += nt) {
+    const LayerCoef &C = sh.L[n];
+    LayerX &X = sh.X[n];
+    X.ns = xdivisor(C.rNS);
+    X.ew = xdivisor(C.rEW);
+    X.up = xdivisor(n > 0 ? sh.L[n - 1].rz : 1.0);
+    X.dn = xdivisor(C.rz);
+    X.edgeNS = xdivisor(C.edgeNS);
+    X.edgeEW = xdivisor(C.edgeEW);
+    X.amb = xdivisor(C.kind == LK_SINK ? C.rz : C.ramb);
+    X.cap = xdivisor(C.cap);
+    X.kind = C.kind;
+    X.base = C.kind == LK_SPREADER ? HSB_SP_W : C.kind == LK_SINK ? HSB_SINK_C_W : C.kind == LK_PCB ? HSB_PCB_C_W
+             : C.kind == LK_SUB ? HSB_SUB_W : HSB_SOLDER_W;
+  }
+  __syncthreads();
   unsigned target = 0;
   int yi = G.yi, ik1 = G.ik1, ik1n = G.ik1n, ik1p = G.ik1p, slot = 0;
   double t = G.t, h = G.h, mx = 0.0;
@@ -302,41 +620,45 @@ __global__ void __launch_bounds__(XT, 1) rk4_exact_kernel(const __grid_constant_
   int status = X_DONE;
   bool have = G.have_k1 != 0;
   for (;;) {
-    XRole r;
-    r.y = G.Y[yi]; r.yn = G.Y[yi ^ 1]; r.t1 = G.t1;
-    r.k1 = G.k[ik1]; r.k1n = G.k[ik1n]; r.k1p = G.k[ik1p];
-    r.Xa0 = G.X[0]; r.Xa1 = G.X[1]; r.Xb0 = G.X[2]; r.Xb1 = G.X[3];
-    r.acca = G.acc[0]; r.accb = G.acc[1];
-    r.h = h;
-    r.hb = h / 2.0;
+    if (tid == 0) {
+      XRole &r = sh.r;
+      r.y = G.Y[yi]; r.yn = G.Y[yi ^ 1]; r.t1 = G.t1;
+      r.k1 = G.k[ik1]; r.k1n = G.k[ik1n]; r.k1p = G.k[ik1p];
+      r.Xa0 = G.X[0]; r.Xa1 = G.X[1]; r.Xb0 = G.X[2]; r.Xb1 = G.X[3];
+      r.acca = G.acc[0]; r.accb = G.acc[1];
+      r.h = h;
+      r.hb = h / 2.0;
+    }
+    __syncthreads();
+    const XRole &r = sh.r;
     const XVec none{nullptr};
     if (!have) {
-      xpass<FIELD, ADV, XP_K1, false>(G, A, sh, xbuf, r, XVec{r.y}, none);
+      xpass<FIELD, ADV, XP_K1, false>(sh, xbuf, XVec{r.y}, none);
       xbarrier(G.bar, target, sh.lost);
     }
     const double rem = G.T - t - h;
     const bool spec = rem >= MIN_STEP * DELTA;   // another step follows this one
-    xpass<FIELD, ADV, XP_1, true>(G, A, sh, xbuf, r, XForm{r.y, r.k1, r.h / 2.0}, XForm{r.y, r.k1, r.hb / 2.0});
+    xpass<FIELD, ADV, XP_1, true>(sh, xbuf, XForm{r.y, r.k1, r.h / 2.0}, XForm{r.y, r.k1, r.hb / 2.0});
     xbarrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_2, true>(G, A, sh, xbuf, r, XVec{r.Xa0}, XVec{r.Xb0});
+    xpass<FIELD, ADV, XP_2, true>(sh, xbuf, XVec{r.Xa0}, XVec{r.Xb0});
     xbarrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_3, true>(G, A, sh, xbuf, r, XVec{r.Xa1}, XVec{r.Xb1});
+    xpass<FIELD, ADV, XP_3, true>(sh, xbuf, XVec{r.Xa1}, XVec{r.Xb1});
     xbarrier(G.bar, target, sh.lost);
-    if (spec) xpass<FIELD, ADV, XP_4S, true>(G, A, sh, xbuf, r, XVec{r.t1}, XVec{r.yn});
-    else xpass<FIELD, ADV, XP_4, false>(G, A, sh, xbuf, r, XVec{r.t1}, none);
+    if (spec) xpass<FIELD, ADV, XP_4S, true>(sh, xbuf, XVec{r.t1}, XVec{r.yn});
+    else xpass<FIELD, ADV, XP_4, false>(sh, xbuf, XVec{r.t1}, none);
     xbarrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_5, false>(G, A, sh, xbuf, r, XVec{r.Xa0}, none);
+    xpass<FIELD, ADV, XP_5, false>(sh, xbuf, XVec{r.Xa0}, none);
     xbarrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_6, false>(G, A, sh, xbuf, r, XVec{r.Xa1}, none);
+    xpass<FIELD, ADV, XP_6, false>(sh, xbuf, XVec{r.Xa1}, none);
     xbarrier(G.bar, target, sh.lost);
-    double err = xpass<FIELD, ADV, XP_7, false>(G, A, sh, xbuf, r, XVec{r.Xa0}, none);
+    double err = xpass<FIELD, ADV, XP_7, false>(sh, xbuf, XVec{r.Xa0}, none);
     for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_down_sync(0xffffffffu, err, o));
     __syncthreads();
     if ((tid & 31) == 0) sh.wmax[tid >> 5] = err;
     __syncthreads();
     if (tid == 0) {
       double m = sh.wmax[0];
-      for (int w = 1; w < XT / 32; w++) m = fmax(m, sh.wmax[w]);
+      for (int w = 1; w < nt / 32; w++) m = fmax(m, sh.wmax[w]);
       atomicMax(G.err + slot, (unsigned long long)__double_as_longlong(m));
     }
     xbarrier(G.bar, target, sh.lost);
@@ -383,15 +705,19 @@ static void fill_packx(const hsb_dev_model *m, PackX *P) {
   const LayerCoef *L = m->hostL0;
   for (int k = 0; k < XNX; k++) {
     P->eidx[k] = -1;
-    P->C[k] = 1.0;
+    P->C[k] = P->edgeR[k] = xdivisor(1.0);
+    for (int q = 0; q < 3; q++) {
+      P->nb[k][q] = k;
+      P->R[k][q] = xdivisor(1.0);
+    }
   }
   auto term = [&](int node, int nb, double R) {
     P->nb[node][P->nt[node]] = nb;
-    P->R[node][P->nt[node]++] = R;
+    P->R[node][P->nt[node]++] = xdivisor(R);
   };
   auto edge = [&](int node, int e, double R) {
     P->eidx[node] = e;
-    P->edgeR[node] = R;
+    P->edgeR[node] = xdivisor(R);
   };
   const int sC[4] = {HSB_SINK_C_N, HSB_SINK_C_S, HSB_SINK_C_W, HSB_SINK_C_E};
   const int sO[4] = {HSB_SINK_N, HSB_SINK_S, HSB_SINK_W, HSB_SINK_E};
@@ -401,15 +727,15 @@ static void fill_packx(const hsb_dev_model *m, PackX *P) {
     const double r2 = (y ? pk.r_hs2_y : pk.r_hs2_x) + pk.r_hs;
     term(sO[s], -1, pk.r_hs_per + pk.r_amb_per);
     term(sO[s], sC[s], r2);
-    P->C[sO[s]] = pk.c_hs_per + pk.c_amb_per;
+    P->C[sO[s]] = xdivisor(pk.c_hs_per + pk.c_amb_per);
     edge(sC[s], s, y ? L[m->hsidx].edgeNS : L[m->hsidx].edgeEW);
     term(sC[s], -1, y ? pk.r_hs_c_per_y + pk.r_amb_c_per_y : pk.r_hs_c_per_x + pk.r_amb_c_per_x);
     term(sC[s], sp[s], y ? pk.r_sp_per_y : pk.r_sp_per_x);
     term(sC[s], sO[s], r2);
-    P->C[sC[s]] = y ? pk.c_hs_c_per_y + pk.c_amb_c_per_y : pk.c_hs_c_per_x + pk.c_amb_c_per_x;
+    P->C[sC[s]] = xdivisor(y ? pk.c_hs_c_per_y + pk.c_amb_c_per_y : pk.c_hs_c_per_x + pk.c_amb_c_per_x);
     edge(sp[s], 4 + s, y ? L[m->spidx].edgeNS : L[m->spidx].edgeEW);
     term(sp[s], sC[s], y ? pk.r_sp_per_y : pk.r_sp_per_x);
-    P->C[sp[s]] = y ? pk.c_sp_per_y : pk.c_sp_per_x;
+    P->C[sp[s]] = xdivisor(y ? pk.c_sp_per_y : pk.c_sp_per_x);
   }
   if (m->nx > HSB_EXTRA) {
     const int pC[4] = {HSB_PCB_C_N, HSB_PCB_C_S, HSB_PCB_C_W, HSB_PCB_C_E};
@@ -421,18 +747,18 @@ static void fill_packx(const hsb_dev_model *m, PackX *P) {
       const double r2 = (y ? pk.r_pcb2_y : pk.r_pcb2_x) + pk.r_pcb;
       term(pO[s], -1, pk.r_amb_sec_per);
       term(pO[s], pC[s], r2);
-      P->C[pO[s]] = pk.c_pcb_per + pk.c_amb_sec_per;
+      P->C[pO[s]] = xdivisor(pk.c_pcb_per + pk.c_amb_sec_per);
       edge(pC[s], 8 + s, y ? L[m->pcbidx].edgeNS : L[m->pcbidx].edgeEW);
       term(pC[s], -1, y ? pk.r_amb_sec_c_per_y : pk.r_amb_sec_c_per_x);
       term(pC[s], so[s], y ? pk.r_pcb_c_per_y : pk.r_pcb_c_per_x);
       term(pC[s], pO[s], r2);
-      P->C[pC[s]] = y ? pk.c_pcb_c_per_y + pk.c_amb_sec_c_per_y : pk.c_pcb_c_per_x + pk.c_amb_sec_c_per_x;
+      P->C[pC[s]] = xdivisor(y ? pk.c_pcb_c_per_y + pk.c_amb_sec_c_per_y : pk.c_pcb_c_per_x + pk.c_amb_sec_c_per_x);
       edge(so[s], 12 + s, y ? L[m->solderidx].edgeNS : L[m->solderidx].edgeEW);
       term(so[s], pC[s], y ? pk.r_pcb_c_per_y : pk.r_pcb_c_per_x);
-      P->C[so[s]] = y ? pk.c_solder_per_y : pk.c_solder_per_x;
+      P->C[so[s]] = xdivisor(y ? pk.c_solder_per_y : pk.c_solder_per_x);
       edge(sb[s], 16 + s, y ? L[m->subidx].edgeNS : L[m->subidx].edgeEW);
       term(sb[s], so[s], y ? pk.r_solder_per_y : pk.r_solder_per_x);
-      P->C[sb[s]] = y ? pk.c_sub_per_y : pk.c_sub_per_x;
+      P->C[sb[s]] = xdivisor(y ? pk.c_sub_per_y : pk.c_sub_per_x);
     }
   }
 }
@@ -443,13 +769,13 @@ static const void *exact_kernel(int v) {
 }
 
 #define XTAIL 512   // barrier counter, error norms and report behind the work vectors
-static_assert(256 + sizeof(XCtl) <= XTAIL, "report fits its place");
+static_assert(256 + sizeof(XCtl) <= XTAIL && sizeof(XCtl) <= HSB_REPORT_BYTES, "report fits its places");
 
 static void free_exact(void *p) {
   XWork *w = (XWork *)p;
   if (!w) return;
   if (w->slab) cudaFree(w->slab);
-  if (w->h_ctl) cudaFreeHost(w->h_ctl);
+  if (w->z) cudaFree(w->z);
   delete w;
 }
 
@@ -460,7 +786,6 @@ static int exact_prepare(hsb_dev_model *m, XWork **out) {
     w = new XWork();
     const size_t vec = ((size_t)m->vlen + 31) / 32 * 32;
     cudaError_t e = cudaMalloc((void **)&w->slab, sizeof(double) * vec * 10 + XTAIL + sizeof(PackX));
-    if (e == cudaSuccess) e = cudaMallocHost((void **)&w->h_ctl, sizeof(XCtl));
     if (e != cudaSuccess) {
       free_exact(w);
       return cuda_check(e, "allocating the transient's work vectors");
@@ -479,6 +804,11 @@ static int exact_prepare(hsb_dev_model *m, XWork **out) {
     PackX P;
     fill_packx(m, &P);
     HSB_CUDA(h2d_on(w->px, &P, sizeof(P), m->stream));
+    if (m->field) {
+      if (!w->z) HSB_CUDA(cudaMalloc((void **)&w->z, sizeof(double) * 7 * m->ncell));
+      xfield_recip<<<(unsigned)((m->ncell + 255) / 256), 256, 0, m->stream>>>(make_args(m, m->L0, m->nr, m->nc), w->z);
+      HSB_CUDA(cudaGetLastError());
+    }
     w->px_version = m->coef_version;
   }
   *out = w;
@@ -490,28 +820,35 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   if (!(0.0 < time_elapsed && h0 >= MIN_STEP * DELTA)) return HSB_OK;   // the loop's own condition
   XWork *w = nullptr;
   int rc;
+  if (m->vlen >= (1LL << 31) - 1) return set_error(HSB_E_NOMEM, "transient: more than 2^31 cells");   // 17 GB a vector
   if ((rc = exact_prepare(m, &w))) return rc;
   const int v = (m->field ? 2 : 0) + (m->uchan_mask ? 1 : 0);
   const void *fn = exact_kernel(v);
   const size_t smem = sizeof(double) * 2 * 40 * (XCHUNK + 1);
-  if (!w->grid[v]) {
+  if (!w->ready[v]) {
     if ((rc = raise_smem_limit(fn, smem))) return rc;
-    int per_sm = 0, nsm = 0;
-    HSB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, m->device));
-    HSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, XT, smem));
-    if (per_sm < 1) return set_error(HSB_E_ARG, "transient kernel does not fit an SM");
-    w->grid[v] = per_sm * nsm;
+    HSB_CUDA(cudaDeviceGetAttribute(&w->nsm, cudaDevAttrMultiProcessorCount, m->device));
+    w->ready[v] = true;
   }
+  // One CTA per SM (148 arrivals at the barrier).  A CTA has as few threads
+  // as give every tile an SM of its own, and XTMAX where the grid is larger
+  // than that and the tiles go round; 256 at least, so that the package CTA's
+  // loads of a 64-cell edge are one batch (128 threads: 306 us at 64x64x4
+  // against 175).
+  int nt = 256;
+  while (nt < XTMAX && (m->ncell + nt - 1) / nt + 1 > w->nsm) nt *= 2;
   XArgs G;
   memset(&G, 0, sizeof(G));
   G.A = make_args(m, m->L0, m->nr, m->nc);
+  G.F.z = w->z;
   G.px = w->px;
   G.el[0] = m->hsidx; G.el[1] = m->spidx; G.el[2] = m->pcbidx; G.el[3] = m->solderidx; G.el[4] = m->subidx;
   int txl = 0;
   while (txl < 5 && (1 << txl) < m->nc) txl++;
   G.txl = txl;
+  while ((1 << G.cwl) < XCHUNK && (1 << G.cwl) < (m->nr > m->nc ? m->nr : m->nc)) G.cwl++;
   G.ntj = (m->nc + (1 << txl) - 1) >> txl;
-  G.nti = (m->nr + (XT >> txl) - 1) / (XT >> txl);
+  G.nti = (m->nr + (nt >> txl) - 1) / (nt >> txl);
   G.tiles = G.ntj * G.nti * m->nl;
   for (int k = 0; k < 3; k++) G.k[k] = w->v[k];
   for (int k = 0; k < 4; k++) G.X[k] = w->v[3 + k];
@@ -523,14 +860,14 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   G.t = 0.0; G.h = h0;
   G.ik1 = 0; G.ik1n = 1; G.ik1p = 2;
   G.Y[0] = m->y; G.Y[1] = m->ytemp;
-  const int grid = w->grid[v] < G.tiles + 1 ? w->grid[v] : G.tiles + 1;
+  const int grid = w->nsm < G.tiles + 1 ? w->nsm : G.tiles + 1;
   for (;;) {
     HSB_CUDA(cudaMemsetAsync(w->bar, 0, XTAIL, m->stream));
     void *args[] = {&G};
-    HSB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(XT), args, smem, m->stream));
-    HSB_CUDA(cudaMemcpyAsync(w->h_ctl, w->ctl, sizeof(XCtl), cudaMemcpyDeviceToHost, m->stream));
+    HSB_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(nt), args, smem, m->stream));
+    XCtl &c = *(XCtl *)m->h_rep;
+    HSB_CUDA(cudaMemcpyAsync(&c, w->ctl, sizeof(XCtl), cudaMemcpyDeviceToHost, m->stream));
     HSB_CUDA(cudaStreamSynchronize(m->stream));
-    const XCtl &c = *w->h_ctl;
     st->launches += 1;
     st->rk4_steps += c.steps;
     st->rk4_attempts += c.attempts;
