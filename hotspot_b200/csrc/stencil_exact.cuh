@@ -9,6 +9,46 @@
 
 namespace hsb {
 
+// x / y for a divisor known in advance, correctly rounded: with zh = RN(1/y)
+// and zl = RN(1/y - zh), q1 = RN(zh x + RN(zl x)) is a faithful quotient
+// (Brisebarre, Muller and Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans.
+// Computers 2004), and one correction with its exact remainder rounds it
+// correctly (Markstein's theorem, IBM J. R&D 1990).  Four multiply-adds in
+// place of a division's reciprocal iteration.  Both proofs need quotients
+// clear of underflow and overflow: `bad` collects results outside 2^-819 ..
+// 2^813 (infinities and NaN included), and the cell is then evaluated with
+// plain divisions.  Zero over anything is exact as it is.
+struct XDiv {
+  double y, zh, zl;
+};
+__device__ __forceinline__ bool xrange_bad(double q, double x) {
+  return ((unsigned)__double2hiint(q) & 0x7fffffffu) - 0x0cc00000u >= 0x66000000u &&
+         ((unsigned)__double2hiint(x) & 0x7fffffffu) != 0u;
+}
+__device__ __forceinline__ double xdiv(double x, const XDiv &d, bool &bad) {
+  const double q1 = __fma_rn(d.zh, x, __dmul_rn(d.zl, x));
+  const double q = __fma_rn(__fma_rn(-d.y, q1, x), d.zh, q1);
+  bad |= xrange_bad(q, x);
+  return q;
+}
+// the same from y and zh alone (per-cell coefficients): the faithful
+// quotient from one more remainder step instead of zl
+__device__ __forceinline__ double xdiv(double x, double y, double zh, bool &bad) {
+  const double q0 = __dmul_rn(x, zh);
+  const double q1 = __fma_rn(__fma_rn(-y, q0, x), zh, q0);
+  const double q = __fma_rn(__fma_rn(-y, q1, x), zh, q1);
+  bad |= xrange_bad(q, x);
+  return q;
+}
+__host__ __device__ inline XDiv xdivisor(double y) {
+  XDiv d;
+  d.y = y;
+  d.zh = 1.0 / y;
+  d.zl = fma(-y, d.zh, 1.0) / y;
+  return d;
+}
+
 // dT/dt of grid cell c = (n,i,j) (temperature_grid.c:3162-3598):
 //   [P + sum_nbr (T_nbr - T)/R + package edges + ambient + advection] / C
 // tv(c) returns the temperature of cell c (or of extra node ncell + k).

@@ -55,3 +55,18 @@ def test_states_outside_the_division_range(workdir, field):
         o.compute_temp(p.copy(), None, 1.5e-7)
         assert np.array_equal(m.grid("trans"), o.grid("trans"), equal_nan=True)
     m.close()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 8), (8, 1), (2, 16), (16, 2), (16, 16), (8, 32)])
+def test_steady_shapes_bit_exact(workdir, rows, cols):
+    """The wavefront sweeps: lines along either direction, single lines and
+    single cells, on every level of the nested iteration."""
+    sc = W.scenario_chip2d(workdir, seed=3 * rows + cols, grid=16, steps=1, n_blocks=1)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    m, o, s, so = _pair(sc)
+    p = m.power_vector(sc.block_power[0])
+    m.steady(p.copy(), s)
+    sweeps = o.steady(p.copy(), so)
+    assert m.stats()["sweeps"] == sweeps
+    assert np.array_equal(s, so) and np.array_equal(m.grid("steady"), o.grid("steady"))
+    m.close()
