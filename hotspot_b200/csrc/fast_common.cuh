@@ -34,6 +34,7 @@ namespace hsb {
 #define FT_MAX_LAYERS 16
 #define PK_LINKS 4
 #define WAIT_LIMIT (1 << 22)  // mbarrier polls before a tile copy is declared lost
+#define FT_CNT_BYTES 256
 #define KRY_DMAX 31           // highest Krylov vector index (six step rejections in a row)
 
 struct LayerF {
@@ -73,7 +74,8 @@ struct FastWork {
   PackF *pk;
   double *part;                   // [2][NEDGE][segmax] edge partial sums
   unsigned long long *err;        // [2] max-norm bits
-  long long *cnt;                 // [0]=steps [1]=attempts [2]=final buffer [3]=status
+  long long *cnt;                 // [0]=steps [1]=attempts [2]=final buffer [3]=status; the paired-pass
+                                  // kernel's barrier counter and error norms behind (FT_CNT_BYTES)
   long long *h_cnt;               // pinned mirror
   Maps maps;
   const double *mapP, *mapQ;      // the state buffers the maps describe
@@ -85,6 +87,9 @@ struct FastWork {
   const void *kfn;                // Krylov kernel variant kgrid was computed for
   int kgrid;                      // its co-resident grid
   cudaEvent_t kev[2];             // kernel timing events
+  bool kmaps;                     // kmap_pf, kmap_N(i) are made
+  double *pair_part;              // edge partial sums of the paired-pass kernel (rk4_pair.cu)
+  int pair_ti, pair_tj;           // its tile (0: not chosen)
   void *tb;                       // temporally blocked kernel's resources (rk4_tb.cu), or null
 };
 

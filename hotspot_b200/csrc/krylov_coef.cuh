@@ -20,29 +20,29 @@ struct Coef {
 // ---------------------------------------------------------------------------
 // coefficient algebra over the basis N_m = (s L)^m F (one thread)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void c_one(Coef &p) {
+__host__ __device__ __forceinline__ void c_one(Coef &p) {
   p.n = 1;
   p.c[0] = 1.0;
 }
-__device__ __forceinline__ void c_copy(Coef &d, const Coef &s) {
+__host__ __device__ __forceinline__ void c_copy(Coef &d, const Coef &s) {
   d.n = s.n;
   for (int j = 0; j < s.n; j++) d.c[j] = s.c[j];
 }
 // w = L v: L N_m = N_{m+1} / s_{m+1}
-__device__ __forceinline__ void c_lop(Coef &w, const Coef &v, const double *ps) {
+__host__ __device__ __forceinline__ void c_lop(Coef &w, const Coef &v, const double *ps) {
   const int n = v.n + 1 < PMAX ? v.n + 1 : PMAX;
   w.c[0] = 0.0;
   for (int j = 1; j < n; j++) w.c[j] = v.c[j - 1] / ps[j];
   w.n = n;
 }
 // y += a x
-__device__ __forceinline__ void c_axpy(Coef &y, double a, const Coef &x) {
+__host__ __device__ __forceinline__ void c_axpy(Coef &y, double a, const Coef &x) {
   for (int j = y.n; j < x.n; j++) y.c[j] = 0.0;
   if (x.n > y.n) y.n = x.n;
   for (int j = 0; j < x.n; j++) y.c[j] += a * x.c[j];
 }
 // y_out - y of rk4_core(y, k1 = K, h) with f(y) = F = N_0 (RCutil.c:440-531)
-__device__ inline void c_core(Coef &out, const Coef &K, double h, const double *s) {
+__host__ __device__ inline void c_core(Coef &out, const Coef &K, double h, const double *s) {
   Coef t, k2, k3, k4;
   c_lop(t, K, s);
   c_one(k2);
@@ -67,7 +67,7 @@ __device__ inline void c_core(Coef &out, const Coef &K, double h, const double *
 
 // the attempt's polynomials (one thread): D = ytemp - y, F1 = f(t1), E = ytemp - t2;
 // vectors not computed yet (index > dcomp) will be made with scale h
-__device__ inline void kry_plan(Coef &E, Coef &D, Coef &F1, const Coef &K, double *ps, double h, int dcomp) {
+static __host__ __device__ __noinline__ void kry_plan(Coef &E, Coef &D, Coef &F1, const Coef &K, double *ps, double h, int dcomp) {
   for (int m = dcomp + 1; m < PMAX; m++) ps[m] = h;
   const double *s = ps;
   Coef dh, d2;

@@ -53,7 +53,6 @@ namespace hsb {
 #define XTMAX 512
 #define XCHUNK 128          // edge cells per chunk of the package CTA
 #define XNX (HSB_EXTRA + HSB_EXTRA_SEC)
-#define XBAR_LIMIT (1 << 22)   // polls before a grid barrier is given up
 
 #define RK4_SAFETY 0.95
 #define RK4_MAXUP 5.0
@@ -109,25 +108,6 @@ struct XWork {
   int nsm;
   bool ready[4];              // per kernel variant: shared memory limit raised
 };
-
-// grid barrier: one arrival per CTA on a counter that only grows
-__device__ __forceinline__ void xbarrier(unsigned *bar, unsigned &target, int &lost) {
-  __syncthreads();
-  target += gridDim.x;
-  if (threadIdx.x == 0 && !lost) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(bar) : "memory");
-    unsigned v;
-    int it = 0;
-    do {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(bar) : "memory");
-      if (++it >= XBAR_LIMIT) {
-        lost = 1;
-        break;
-      }
-    } while ((int)(v - target) < 0);
-  }
-  __syncthreads();
-}
 
 // stage inputs: a stored vector, or y + a k formed on the fly
 struct XVec {
@@ -595,23 +575,23 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
     const XVec none{nullptr};
     if (!have) {
       xpass<FIELD, ADV, XP_K1, false>(sh, xbuf, XVec{r.y}, none);
-      xbarrier(G.bar, target, sh.lost);
+      grid_barrier(G.bar, target, sh.lost);
     }
     const double rem = G.T - t - h;
     const bool spec = rem >= MIN_STEP * DELTA;   // another step follows this one
     xpass<FIELD, ADV, XP_1, true>(sh, xbuf, XForm{r.y, r.k1, r.h / 2.0}, XForm{r.y, r.k1, r.hb / 2.0});
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     xpass<FIELD, ADV, XP_2, true>(sh, xbuf, XVec{r.Xa0}, XVec{r.Xb0});
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     xpass<FIELD, ADV, XP_3, true>(sh, xbuf, XVec{r.Xa1}, XVec{r.Xb1});
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     if (spec) xpass<FIELD, ADV, XP_4S, true>(sh, xbuf, XVec{r.t1}, XVec{r.yn});
     else xpass<FIELD, ADV, XP_4, false>(sh, xbuf, XVec{r.t1}, none);
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     xpass<FIELD, ADV, XP_5, false>(sh, xbuf, XVec{r.Xa0}, none);
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     xpass<FIELD, ADV, XP_6, false>(sh, xbuf, XVec{r.Xa1}, none);
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     double err = xpass<FIELD, ADV, XP_7, false>(sh, xbuf, XVec{r.Xa0}, none);
     for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_down_sync(0xffffffffu, err, o));
     __syncthreads();
@@ -622,7 +602,7 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
       for (int w = 1; w < nt / 32; w++) m = fmax(m, sh.wmax[w]);
       atomicMax(G.err + slot, (unsigned long long)__double_as_longlong(m));
     }
-    xbarrier(G.bar, target, sh.lost);
+    grid_barrier(G.bar, target, sh.lost);
     mx = __longlong_as_double((long long)*(volatile unsigned long long *)(G.err + slot));
     slot ^= 1;
     if (blockIdx.x == 0 && tid == 0) G.err[slot] = 0ull;

@@ -582,7 +582,7 @@ static void free_fast(void *p) {
   if (!w) return;
   void *bufs[] = {w->k1, w->k2, w->k3, w->pf, w->ytemp, w->t1, w->t2, w->gN, w->gS, w->gW, w->gE,
                   w->gA, w->gB, w->invC, w->aN, w->aS, w->aW, w->aE, w->aO, w->Lf, w->pk, w->part,
-                  w->err, w->cnt, w->N};
+                  w->err, w->cnt, w->N, w->pair_part};
   for (void *b : bufs)
     if (b) cudaFree(b);
   if (w->h_cnt) cudaFreeHost(w->h_cnt);
@@ -626,7 +626,7 @@ int fast_prepare(hsb_dev_model *m, FastWork **out) {
     HSB_CUDA(cudaMalloc(&w->pk, sizeof(PackF)));
     HSB_CUDA(cudaMalloc(&w->part, sizeof(double) * 2 * NEDGE * w->segmax));
     HSB_CUDA(cudaMalloc(&w->err, sizeof(unsigned long long) * 2));
-    HSB_CUDA(cudaMalloc(&w->cnt, sizeof(long long) * 8));
+    HSB_CUDA(cudaMalloc(&w->cnt, FT_CNT_BYTES));
     HSB_CUDA(cudaMallocHost(&w->h_cnt, sizeof(long long) * 8));
   }
   // the maps describe the two state buffers whichever role each has now

@@ -34,6 +34,7 @@
 
 #include "fast_common.cuh"
 #include "krylov_coef.cuh"
+#include "rk4_pair.cuh"
 #include "rk4_tb.cuh"
 
 namespace cg = cooperative_groups;
@@ -708,7 +709,12 @@ int kry_prepare(hsb_dev_model *m, FastWork *w) {
     if (!tb) return set_error(HSB_E_ARG, "the blocked forms take models with per-layer conductances and 3..12 layers");
     return tb_prepare_single(m, w);
   }
-  if (m->fast_passes == 0 && tb && m->ncell >= TB_MIN_CELLS) return tb_prepare_single(m, w);
+  if (m->fast_passes == 0) {
+    if (tb && m->ncell >= TB_MIN_CELLS) return tb_prepare_single(m, w);
+    bool taken = false;
+    const int rc = pair_prepare(m, w, &taken);
+    if (rc || taken) return rc;
+  }
   return kry_prepare_vectors(m, w);
 }
 
@@ -718,9 +724,12 @@ int kry_prepare_vectors(hsb_dev_model *m, FastWork *w) {
   if (!w->N) {
     w->nstride = (m->ncell + 63) / 64 * 64;
     HSB_CUDA(cudaMalloc(&w->N, sizeof(float) * w->nstride * (KRY_DMAX + 1)));
+  }
+  if (!w->kmaps) {
     if ((rc = make_map(&w->kmap_pf, w->pf, false, m, TJ, TI))) return rc;
     if ((rc = make_map4(&w->kmap_N, w->N, m, KW, HR, KRY_DMAX + 1, w->nstride))) return rc;
     if ((rc = make_map4(&w->kmap_Ni, w->N, m, TJ, TI, KRY_DMAX + 1, w->nstride))) return rc;
+    w->kmaps = true;
   }
   if (w->kmap_ybuf == w->ytemp && w->kmap_y2buf == m->y) {   // the buffers swapped roles: swap their maps
     CUtensorMap t = w->kmap_y;
@@ -802,6 +811,7 @@ int rk4_krylov_enqueue(hsb_dev_model *m, FastWork *w, double T, hsb_stats *st, c
   int rc;
   if ((rc = kry_prepare(m, w))) return rc;
   if (w->kfn == tb_kernel(false) || w->kfn == tb_kernel(true)) return tb_enqueue(m, w, T, st, bpow, K);
+  if (pair_is_kernel(w->kfn)) return pair_enqueue(m, w, T, st, bpow, K);
   KryArgs A;
   memset(&A, 0, sizeof(A));
   A.m_y = w->kmap_y;

@@ -9,6 +9,34 @@
 
 namespace hsb {
 
+#define HSB_BAR_LIMIT (1 << 22)   // polls before a grid barrier is given up
+// grid barrier of a cooperative launch: one arrival per CTA on a counter that
+// only grows (2.1 thousand cycles over 148 CTAs of a B200)
+// In two halves: a CTA's threads may work between them.
+__device__ __forceinline__ void grid_arrive(unsigned *bar, unsigned &target, int &lost) {
+  __syncthreads();
+  target += gridDim.x;
+  if (threadIdx.x == 0 && !lost) asm volatile("red.release.gpu.global.add.u32 [%0], 1;\n" ::"l"(bar) : "memory");
+}
+__device__ __forceinline__ void grid_wait(unsigned *bar, unsigned target, int &lost) {
+  if (threadIdx.x == 0 && !lost) {
+    unsigned v;
+    int it = 0;
+    do {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(v) : "l"(bar) : "memory");
+      if (++it >= HSB_BAR_LIMIT) {
+        lost = 1;
+        break;
+      }
+    } while ((int)(v - target) < 0);
+  }
+  __syncthreads();
+}
+__device__ __forceinline__ void grid_barrier(unsigned *bar, unsigned &target, int &lost) {
+  grid_arrive(bar, target, lost);
+  grid_wait(bar, target, lost);
+}
+
 // x / y for a divisor known in advance, correctly rounded: with zh = RN(1/y)
 // and zl = RN(1/y - zh), q1 = RN(zh x + RN(zl x)) is a faithful quotient
 // (Brisebarre, Muller and Raina, "Accelerating correctly rounded

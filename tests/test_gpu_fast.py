@@ -10,7 +10,7 @@ direct LU, bar max |dT| <= 0.01 K (the solver converges far below it).
 import numpy as np
 import pytest
 
-from hotspot_b200 import FORM_FAST
+from hotspot_b200 import FORM_FAST, FORM_FAST_PASSES
 from hotspot_b200 import model as hm
 from hotspot_b200 import workloads as W
 from oracle.restatement import OracleModel
@@ -236,3 +236,33 @@ def test_mg_steady_secondary_path(workdir):
     (sf, gf, stf), (sr, gr, _) = out
     assert np.max(np.abs(sf - sr)) <= TOL and np.max(np.abs(gf - gr)) <= TOL
     assert stf["residual"] < 1e-6
+
+
+@pytest.mark.parametrize("rows,cols,dt", [(4, 8, 3.333e-6), (8, 4, 3.333e-6), (16, 256, 1e-5), (256, 16, 1e-5), (64, 128, 2e-3),
+                                          (128, 64, 3.333e-6)])
+def test_paired_passes_shapes(workdir, rows, cols, dt):
+    """The paired-pass transient kernel at the edges of its tiles: grids
+    smaller than a tile, tiles along one edge only, long intervals with
+    rejected attempts, and a trace of intervals in one launch against the
+    same intervals one by one.  Bar: the fast form's (0.01 K); the steps are
+    those of the same arithmetic one pass at a time (FP32 error norms need not
+    take the FP64 steps on long intervals)."""
+    sc = W.scenario_stack3d(workdir, seed=rows + cols, grid=16, steps=3, n_blocks=3)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    m, n, q, o = hm.from_scenario(sc), hm.from_scenario(sc), hm.from_scenario(sc), OracleModel(sc)
+    m.set_solver(FORM_FAST)
+    q.set_solver(FORM_FAST_PASSES)
+    t, to, tq = m.vector(o.init_temp), o.vector(o.init_temp), m.vector(o.init_temp)
+    ps = np.stack([m.power_vector(sc.block_power[k]) for k in range(sc.steps)])
+    for k in range(sc.steps):
+        m.compute_temp(ps[k].copy(), t if k == 0 else None, dt)
+        q.compute_temp(ps[k].copy(), tq if k == 0 else None, dt)
+        o.compute_temp(ps[k].copy(), to if k == 0 else None, dt)
+        a, b = m.stats(), q.stats()
+        assert (a["rk4_steps"], a["rk4_attempts"], a["slope_evals"]) == (b["rk4_steps"], b["rk4_attempts"], b["slope_evals"])
+    assert m.transient_kernel() == "passes"
+    assert np.max(np.abs(m.grid("trans") - o.grid("trans"))) <= TOL
+    tn, _ = n.compute_trace(ps, n.vector(o.init_temp), dt, form=FORM_FAST)
+    assert np.array_equal(n.grid("trans"), m.grid("trans")) and np.array_equal(tn, t)
+    for x in (m, n, q):
+        x.close()
