@@ -71,6 +71,8 @@ struct MgLevel {
   float *pinv;                 // NXP x NXP inverse of the package block at this level
 };
 
+struct MgUniform;                // the per-layer models' iteration (mg_uniform.cuh)
+
 struct MgWork {
   int nlev, coef_version;
   std::vector<MgLevel> lv;
@@ -101,6 +103,8 @@ struct MgWork {
   int fuse;
   size_t fuse_smem;
   unsigned *dot_ticket;          // last-block counter of dot_one (returns to 0 after each launch)
+  bool field;                    // the per-cell operators' arrays are allocated
+  MgUniform *u;                  // set while the model's operator is per layer
 };
 
 // ---------------------------------------------------------------------------
@@ -994,17 +998,24 @@ __global__ void pcg_update_p(float *__restrict__ p, const float *__restrict__ z,
   p[k] = z[k] + beta * p[k];
 }
 
-// T += e; the max |e| (K) into *emax_bits (zeroed by the caller)
-__global__ void add_correction(double *__restrict__ T, const float *__restrict__ e, long long n,
-                               unsigned long long *emax_bits) {
-  long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// T += e; the max |e| (K) into *emax_bits (zeroed by the caller), one atomic
+// per CTA (one per warp was most of the time on large grids)
+__global__ void __launch_bounds__(MGT) add_correction(double *__restrict__ T, const float *__restrict__ e, long long n,
+                                                      unsigned long long *emax_bits) {
+  __shared__ double wm[MGT / 32];
   double a = 0.0;
-  if (k < n) {
-    T[k] += (double)e[k];
-    a = fabs((double)e[k]);
+  for (long long k = (long long)blockIdx.x * MGT + threadIdx.x; k < n; k += (long long)gridDim.x * MGT) {
+    const double d = (double)e[k];
+    T[k] += d;
+    a = fmax(a, fabs(d));
   }
   for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_down_sync(0xffffffffu, a, o));
-  if ((threadIdx.x & 31) == 0 && a > 0.0) atomicMax(emax_bits, (unsigned long long)__double_as_longlong(a));
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = a;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < MGT / 32; w++) a = fmax(a, wm[w]);
+    if (a > 0.0) atomicMax(emax_bits, (unsigned long long)__double_as_longlong(a));
+  }
 }
 
 __global__ void copy_f(const float *__restrict__ a, float *__restrict__ b, long long n) {
@@ -1070,6 +1081,12 @@ __global__ void d2f(const double *__restrict__ a, float *__restrict__ b, long lo
   if (k < n) b[k] = (float)a[k];
 }
 
+}  // namespace hsb
+
+#include "mg_uniform.cuh"
+
+namespace hsb {
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1098,6 +1115,132 @@ static MgLevelDev dev_level(const hsb_dev_model *m, const MgLevel &L, int lvl) {
 }
 
 static void free_mg(void *p);
+
+// ---------------------------------------------------------------------------
+// per-layer models: mg_uniform.cuh's kernels
+// ---------------------------------------------------------------------------
+#define MGU_TICKETS 16
+struct MgUniform {
+  int nlev, small;             // levels small .. nlev - 1 run in mgu_small
+  ULev L[24];
+  ULev64 L64;
+  float *tab;                  // all levels' tables
+  float *epart, *esum;         // edge sums: the tiles' shares, the levels' of x after pre-smoothing
+  int seg;
+  double *part;
+  unsigned *ticket;            // one per kernel of an iteration that has a last CTA
+  float *p2;                   // the search direction's second buffer
+  int *par;
+  size_t small_smem;
+  bool pcg;                    // the whole pass in mgu_small
+};
+
+template <int NL, bool PCG>
+static int u_launch_small(hsb_dev_model *m, const MgUniform &u, const USmall &S) {
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(MGU_CL);
+  cfg.blockDim = dim3(MGU_ST);
+  cfg.dynamicSmemBytes = u.small_smem;
+  cfg.stream = m->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = MGU_CL;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  HSB_CUDA(cudaLaunchKernelEx(&cfg, mgu_small<NL, PCG>, S));
+  return HSB_OK;
+}
+
+// z = V-cycle(r), with (r, z) into sc[2]; then q = A p and (p, q), e and r.
+// Models within mgu_small: all n_it iterations at once.
+template <int NL>
+static int u_iteration(hsb_dev_model *m, MgWork *w, int it, int n_it) {
+  MgUniform &u = *w->u;
+  const int c = u.small;
+  double *sc = w->red;
+  USmall S;
+  memset(&S, 0, sizeof(S));
+  S.nlev = u.nlev - c;
+  for (int k = 0; k < S.nlev; k++) S.L[k] = u.L[c + k];
+  S.ps = w->d_ps;
+  S.cinv = w->cinv;
+  S.cn = w->cn;
+  S.tabs = u.L[c].tab;
+  if (u.pcg) {
+    S.f = w->rr;
+    S.out = w->e;
+    S.iters = n_it;
+    return u_launch_small<NL, true>(m, u, S);
+  }
+  auto grid = [&](const ULev &L) { return dim3((L.nc + MGU_TC - 1) / MGU_TC, (L.nr + MGU_TR - 1) / MGU_TR); };
+  auto f_of = [&](int l) { return l == 0 ? w->rr : w->lv[l].f; };
+  const size_t s_down = sizeof(float) * NL * (U_H2 * U_W2 + U_H1 * U_W1), s_post = sizeof(float) * NL * U_H2 * U_W2;
+  unsigned *tk = u.ticket;
+  for (int l = 0; l < c; l++) {
+    mgu_pre<NL><<<grid(u.L[l]), MGU_T, 0, m->stream>>>(u.L[l], w->d_ps, f_of(l), w->lv[l].x, u.epart, u.seg,
+                                                              u.esum + 20 * l, tk);
+    mgu_down<NL><<<grid(u.L[l]), MGU_T, s_down, m->stream>>>(u.L[l], m->nx, f_of(l), w->lv[l].x, w->lv[l + 1].f);
+  }
+  S.f = f_of(c);
+  S.out = w->lv[c].r;
+  S.F = u.L[c - 1];
+  S.ff = f_of(c - 1);
+  S.esum = u.esum + 20 * (c - 1);
+  S.xpf = w->lv[c - 1].x + w->lv[c - 1].ncell;
+  const int rc = u_launch_small<NL, false>(m, u, S);
+  if (rc) return rc;
+  for (int l = c - 1; l >= 0; l--) {
+    const float *xp = w->lv[l].x + w->lv[l].ncell;
+    if (l > 0)
+      mgu_post<NL, false><<<grid(u.L[l]), MGU_T, s_post, m->stream>>>(
+          u.L[l], w->d_ps, f_of(l), w->lv[l].x, w->lv[l + 1].r, xp, w->lv[l].r, tk, u.L[l - 1], f_of(l - 1),
+          u.epart, u.seg, u.esum + 20 * (l - 1), w->lv[l - 1].x + w->lv[l - 1].ncell, nullptr, nullptr);
+    else
+      mgu_post<NL, true><<<grid(u.L[l]), MGU_T, s_post, m->stream>>>(u.L[l], w->d_ps, f_of(l), w->lv[l].x,
+                                                                     w->lv[l + 1].r, xp, w->z, tk, u.L[l], nullptr,
+                                                                     u.epart, u.seg, nullptr, nullptr, u.part, sc);
+  }
+  mgu_apply<NL><<<grid(u.L[0]), MGU_T, 0, m->stream>>>(u.L[0], w->d_ps, w->z, w->p, u.p2, u.par, w->q, u.epart,
+                                                       u.seg, u.part, sc, tk,
+                                                       it == 0);
+  const long long n = w->lv[0].n;
+  mgu_step<<<(unsigned)((n / 4 + 256) / 256), 256, 0, m->stream>>>(w->e, w->rr, w->p, u.p2, u.par, w->q, sc, n, it == 0);
+  return HSB_OK;
+}
+
+#define U_DISPATCH(nl, call)                                                                           \
+  switch (nl) {                                                                                        \
+    case 3: call(3); break;  case 4: call(4); break;  case 5: call(5); break;  case 6: call(6); break; \
+    case 7: call(7); break;  case 8: call(8); break;  case 9: call(9); break;                          \
+    case 10: call(10); break; case 11: call(11); break; case 12: call(12); break;                      \
+  }
+
+static int u_iter(hsb_dev_model *m, MgWork *w, int it, int n_it) {
+  int rc = HSB_OK;
+#define U_CALL(N) rc = u_iteration<N>(m, w, it, n_it)
+  U_DISPATCH(m->nl, U_CALL)
+#undef U_CALL
+  return rc;
+}
+
+static int u_small_setup(int nl, size_t smem, bool pcg) {
+  const void *fn = nullptr;
+#define U_CALL(N) fn = pcg ? (const void *)mgu_small<N, true> : (const void *)mgu_small<N, false>
+  U_DISPATCH(nl, U_CALL)
+#undef U_CALL
+  HSB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  return raise_smem_limit(fn, smem);
+}
+
+static void u_free(MgUniform *u) {
+  if (!u) return;
+  void *b[] = {u->tab, u->epart, u->part, u->ticket, u->p2};
+  for (void *q : b)
+    if (q) cudaFree(q);
+  delete u;
+}
 
 // workspace arrays start zeroed: no kernel of the solver depends on what an
 // earlier allocation left in the memory it reuses.  The zeroing is ordered
@@ -1130,10 +1273,6 @@ static int mg_setup(hsb_dev_model *m, MgWork **out) {
   w->nlev = (int)w->lv.size();
   for (int l = 0; l < w->nlev; l++) {
     MgLevel &L = w->lv[l];
-    HSB_CUDA(mg_alloc(&L.gE, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.gS, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.gB, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.diag, sizeof(float) * L.ncell, m->stream));
     HSB_CUDA(mg_alloc(&L.gAmbL, sizeof(float) * HSB_MAX_LAYERS, m->stream));
     HSB_CUDA(mg_alloc(&L.gEdgeNS, sizeof(float) * HSB_MAX_LAYERS, m->stream));
     HSB_CUDA(mg_alloc(&L.gEdgeEW, sizeof(float) * HSB_MAX_LAYERS, m->stream));
@@ -1142,14 +1281,10 @@ static int mg_setup(hsb_dev_model *m, MgWork **out) {
     HSB_CUDA(mg_alloc(&L.r, sizeof(float) * L.n, m->stream));
     HSB_CUDA(mg_alloc(&L.pinv, sizeof(float) * NXP * NXP, m->stream));
   }
-  const long long n0 = w->lv[0].n, ncell = m->ncell;
-  HSB_CUDA(mg_alloc(&w->gE64, sizeof(double) * ncell, m->stream));
-  HSB_CUDA(mg_alloc(&w->gS64, sizeof(double) * ncell, m->stream));
-  HSB_CUDA(mg_alloc(&w->gB64, sizeof(double) * ncell, m->stream));
+  const long long n0 = w->lv[0].n;
   HSB_CUDA(mg_alloc(&w->gAmb64, sizeof(double) * (HSB_MAX_LAYERS + 3 * NXP + NXP * NXP), m->stream));
   HSB_CUDA(mg_alloc(&w->gEdgeNS64, sizeof(double) * HSB_MAX_LAYERS, m->stream));
   HSB_CUDA(mg_alloc(&w->gEdgeEW64, sizeof(double) * HSB_MAX_LAYERS, m->stream));
-  HSB_CUDA(mg_alloc(&w->r64, sizeof(double) * n0, m->stream));
   HSB_CUDA(mg_alloc(&w->b64, sizeof(double) * n0, m->stream));
   HSB_CUDA(mg_alloc(&w->p, sizeof(float) * n0, m->stream));
   HSB_CUDA(mg_alloc(&w->q, sizeof(float) * n0, m->stream));
@@ -1166,9 +1301,27 @@ static int mg_setup(hsb_dev_model *m, MgWork **out) {
   return HSB_OK;
 }
 
+// the per-cell operators' arrays, for models that need them
+static int mg_alloc_field(hsb_dev_model *m, MgWork *w) {
+  if (w->field) return HSB_OK;
+  for (auto &L : w->lv) {
+    HSB_CUDA(mg_alloc(&L.gE, sizeof(float) * L.ncell, m->stream));
+    HSB_CUDA(mg_alloc(&L.gS, sizeof(float) * L.ncell, m->stream));
+    HSB_CUDA(mg_alloc(&L.gB, sizeof(float) * L.ncell, m->stream));
+    HSB_CUDA(mg_alloc(&L.diag, sizeof(float) * L.ncell, m->stream));
+  }
+  HSB_CUDA(mg_alloc(&w->gE64, sizeof(double) * m->ncell, m->stream));
+  HSB_CUDA(mg_alloc(&w->gS64, sizeof(double) * m->ncell, m->stream));
+  HSB_CUDA(mg_alloc(&w->gB64, sizeof(double) * m->ncell, m->stream));
+  HSB_CUDA(mg_alloc(&w->r64, sizeof(double) * w->lv[0].n, m->stream));
+  w->field = true;
+  return HSB_OK;
+}
+
 static void free_mg(void *p) {
   MgWork *w = (MgWork *)p;
   if (!w) return;
+  u_free(w->u);
   for (auto &L : w->lv) {
     float *b[] = {L.gE, L.gS, L.gB, L.diag, L.gAmbL, L.gEdgeNS, L.gEdgeEW, L.x, L.f, L.r, L.pinv};
     for (float *q : b)
@@ -1186,13 +1339,151 @@ static void free_mg(void *p) {
   delete w;
 }
 
+// level l of a per-layer model (its conductances as mg_coarsen would give them:
+// lateral ones stay, vertical and ambient ones grow with the cell, edge ones
+// with its width)
+static ULev u_level(const hsb_dev_model *m, const MgWork *w, int l, const double *gamb, const double *gens,
+                    const double *geew) {
+  ULev L;
+  memset(&L, 0, sizeof(L));
+  L.nr = w->lv[l].nr;
+  L.nc = w->lv[l].nc;
+  L.nl = m->nl;
+  const float m4 = (float)(1ll << (2 * l));
+  for (int n = 0; n < m->nl; n++) {
+    const LayerCoef &c = m->hostL0[n];
+    L.gE[n] = (float)(1.0 / c.rEW);
+    L.gS[n] = (float)(1.0 / c.rNS);
+    L.gB[n] = n < m->nl - 1 ? (float)(1.0 / c.rz) * m4 : 0.f;
+    L.gAmb[n] = (float)(gamb[n] * (double)m4);
+    L.gNS[n] = (float)(gens[n] * (double)(1ll << l));
+    L.gEW[n] = (float)(geew[n] * (double)(1ll << l));
+    L.base[n] = c.kind == LK_SINK ? HSB_SINK_C_W : c.kind == LK_SPREADER ? HSB_SP_W : c.kind == LK_PCB ? HSB_PCB_C_W
+                : c.kind == LK_SOLDER ? HSB_SOLDER_W : c.kind == LK_SUB ? HSB_SUB_W : -1;
+  }
+  L.nx = m->nx;
+  L.scale = (float)(1 << l);
+  edge_layers(m, L.el);
+  L.ne = m->nx > HSB_EXTRA ? 20 : 8;
+  for (int k = 0; k < NXP; k++) {
+    L.eidx[k] = -1;
+    for (int g = 0; g < 5; g++)
+      if (k < m->nx && w->ps.elayer[k] >= 0 && w->ps.elayer[k] == L.el[g]) L.eidx[k] = (signed char)(4 * g + w->ps.eside[k]);
+  }
+  return L;
+}
+
+// the diagonal of a cell (mg_diag's order)
+static float u_diag(const ULev &L, int n, bool i0, bool i1, bool j0, bool j1) {
+  float d = L.gAmb[n];
+  if (!j1) d += L.gE[n];
+  if (!j0) d += L.gE[n];
+  if (!i1) d += L.gS[n];
+  if (!i0) d += L.gS[n];
+  if (n < L.nl - 1) d += L.gB[n];
+  if (n > 0) d += L.gB[n - 1];
+  if (L.base[n] >= 0) {
+    if (i0) d += L.gNS[n];
+    if (i1) d += L.gNS[n];
+    if (j0) d += L.gEW[n];
+    if (j1) d += L.gEW[n];
+  }
+  return d;
+}
+
+// the per-layer models' tables and buffers; w->u stays null where the small
+// levels do not fit
+static int u_build(hsb_dev_model *m, MgWork *w, const double *gamb, const double *gens, const double *geew,
+                   const std::vector<float> &pinv) {
+  const int nl = m->nl;
+  if (!w->u) {
+    // the finest level from which on everything fits mgu_small
+    int c = 0;
+    size_t smem = 0;
+    bool pcg = false;
+    for (; c < w->nlev; c++) {
+      const MgLevel &L = w->lv[c];
+      if (L.plane > MGU_SMALL || w->nlev - c > MGU_SLEV || u_strip(L.nr, L.nc) * (L.nc / 2) > MGU_ST) continue;
+      USmall S;
+      memset(&S, 0, sizeof(S));
+      S.nlev = w->nlev - c;
+      S.cn = w->cn;
+      for (int k = 0; k < S.nlev; k++) S.L[k] = u_level(m, w, c + k, gamb, gens, geew);
+      pcg = c == 0;
+      smem = sizeof(float) * u_small_floats(S, nl, m->nx, pcg);
+      if (smem <= 200 * 1024) break;
+    }
+    if (c == w->nlev || w->nlev > 24) return HSB_OK;
+    MgUniform *u = new MgUniform();
+    memset(u, 0, sizeof(*u));
+    u->nlev = w->nlev;
+    u->small = c;
+    u->pcg = pcg;
+    u->small_smem = smem;
+    const size_t blocks = (size_t)((m->nc + MGU_TC - 1) / MGU_TC) * ((m->nr + MGU_TR - 1) / MGU_TR);
+    w->u = u;
+    u->seg = std::max((m->nc + MGU_TC - 1) / MGU_TC, (m->nr + MGU_TR - 1) / MGU_TR);
+    HSB_CUDA(mg_alloc(&u->tab, sizeof(float) * w->nlev * u_tab_floats(nl, m->nx), m->stream));
+    HSB_CUDA(mg_alloc(&u->epart, sizeof(float) * 20 * (u->seg + w->nlev), m->stream));
+    u->esum = u->epart + 20 * u->seg;
+    HSB_CUDA(mg_alloc(&u->part, sizeof(double) * blocks, m->stream));
+    HSB_CUDA(mg_alloc(&u->ticket, 64, m->stream));
+    HSB_CUDA(mg_alloc(&u->p2, sizeof(float) * w->lv[0].n, m->stream));
+    u->par = (int *)(u->ticket + 8);
+    int rc;
+    if ((rc = u_small_setup(nl, u->small_smem, u->pcg))) return rc;
+  }
+  MgUniform &u = *w->u;
+  const size_t tf = u_tab_floats(nl, m->nx);
+  std::vector<float> tab(w->nlev * tf);
+  for (int l = 0; l < w->nlev; l++) {
+    ULev &L = u.L[l];
+    L = u_level(m, w, l, gamb, gens, geew);
+    L.tab = u.tab + l * tf;
+    for (int k = 0; k < m->nx; k++)
+      for (int o = 0; o < m->nx; o++) tab[l * tf + 18 * nl + k * m->nx + o] = pinv[((size_t)l * NXP + k) * NXP + o];
+    for (int q = 0; q < 9; q++) {
+      float *t = tab.data() + l * tf + (size_t)q * nl * 2;
+      const int a = q / 3, b = q % 3;
+      float c = 0.f;
+      for (int n = 0; n < nl; n++) {
+        const float d = u_diag(L, n, a == 0, a == 2 || L.nr == 1, b == 0, b == 2 || L.nc == 1);
+        const float iv = 1.f / (n > 0 ? d - L.gB[n - 1] * c : d);
+        c = L.gB[n] * iv;
+        t[2 * n] = iv;
+        t[2 * n + 1] = c;
+      }
+    }
+  }
+  HSB_CUDA(h2d_on(u.tab, tab.data(), sizeof(float) * tab.size(), m->stream));
+  ULev64 &D = u.L64;
+  memset(&D, 0, sizeof(D));
+  D.nr = m->nr; D.nc = m->nc; D.nl = nl; D.nx = m->nx;
+  for (int n = 0; n < nl; n++) {
+    const LayerCoef &c = m->hostL0[n];
+    D.gE[n] = 1.0 / c.rEW;
+    D.gS[n] = 1.0 / c.rNS;
+    D.gB[n] = n < nl - 1 ? 1.0 / c.rz : 0.0;
+    D.gAmb[n] = gamb[n];
+    D.gNS[n] = gens[n];
+    D.gEW[n] = geew[n];
+    D.base[n] = u.L[0].base[n];
+  }
+  return HSB_OK;
+}
+
 // build level operators from the device model's current conductances
 static int mg_build(hsb_dev_model *m, MgWork *w) {
   const StencilArgs S = make_args(m, m->L0, m->nr, m->nc);
   const int nl = m->nl;
   const package_RC_t &pk = m->h_pk;
-  // FP64 fine faces
-  if (m->field) field_faces64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64);
+  // per-layer models have mg_uniform.cuh's kernels; the others FP64 fine faces
+  const bool uni = !m->field && nl >= MGU_MINL && nl <= MGU_MAXL;
+  std::vector<float> pinvs;      // of every level, for the per-layer models' tables
+  int rc0;
+  if (!uni && (rc0 = mg_alloc_field(m, w))) return rc0;
+  if (uni) {
+  } else if (m->field) field_faces64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64);
   else uniform_faces64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64);
   // per-layer ambient and edge conductances (FP64 and per level FP32): the
   // sink's and, on the secondary path, the PCB's cells to ambient; the edge
@@ -1300,6 +1591,7 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
     float inv32[NXP * NXP];
     for (int a = 0; a < NXP; a++)
       for (int o = 0; o < NXP; o++) inv32[a * NXP + o] = (float)M[a][NXP + o];
+    if (uni) pinvs.insert(pinvs.end(), inv32, inv32 + NXP * NXP);
     HSB_CUDA(h2d_on(L.pinv, inv32, sizeof(inv32), m->stream));
   }
   double pack64[HSB_MAX_LAYERS + 3 * NXP + NXP * NXP];
@@ -1323,6 +1615,7 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
     HSB_CUDA(cudaMemcpyAsync(L.gAmbL, ga, sizeof(float) * nl, cudaMemcpyHostToDevice, m->stream));
     HSB_CUDA(cudaMemcpyAsync(L.gEdgeNS, gn, sizeof(float) * nl, cudaMemcpyHostToDevice, m->stream));
     HSB_CUDA(cudaMemcpyAsync(L.gEdgeEW, ge, sizeof(float) * nl, cudaMemcpyHostToDevice, m->stream));
+    if (uni) continue;
     if (l == 0) {
       d2f<<<nb(L.ncell), MGT, 0, m->stream>>>(w->gE64, L.gE, L.ncell);
       d2f<<<nb(L.ncell), MGT, 0, m->stream>>>(w->gS64, L.gS, L.ncell);
@@ -1349,11 +1642,22 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
     w->cn = 0;
     if (n <= MG_COARSE_MAX) {
       std::vector<float> gE(C.ncell), gS(C.ncell), gB(C.ncell), dg(C.ncell);
-      HSB_CUDA(cudaMemcpyAsync(gE.data(), C.gE, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
-      HSB_CUDA(cudaMemcpyAsync(gS.data(), C.gS, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
-      HSB_CUDA(cudaMemcpyAsync(gB.data(), C.gB, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
-      HSB_CUDA(cudaMemcpyAsync(dg.data(), C.diag, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
-      HSB_CUDA(cudaStreamSynchronize(m->stream));
+      if (uni) {
+        const ULev L = u_level(m, w, lc, gamb, gens, geew);
+        for (long long c = 0; c < C.ncell; c++) {
+          const int ln = (int)(c / C.plane), q = (int)(c - ln * C.plane), i = q / C.nc, j = q - i * C.nc;
+          gE[c] = j < C.nc - 1 ? L.gE[ln] : 0.f;
+          gS[c] = i < C.nr - 1 ? L.gS[ln] : 0.f;
+          gB[c] = L.gB[ln];
+          dg[c] = u_diag(L, ln, i == 0, i == C.nr - 1, j == 0, j == C.nc - 1);
+        }
+      } else {
+        HSB_CUDA(cudaMemcpyAsync(gE.data(), C.gE, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
+        HSB_CUDA(cudaMemcpyAsync(gS.data(), C.gS, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
+        HSB_CUDA(cudaMemcpyAsync(gB.data(), C.gB, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
+        HSB_CUDA(cudaMemcpyAsync(dg.data(), C.diag, sizeof(float) * C.ncell, cudaMemcpyDeviceToHost, m->stream));
+        HSB_CUDA(cudaStreamSynchronize(m->stream));
+      }
       const double scale = (double)(1ll << lc);
       std::vector<double> A((size_t)n * 2 * n, 0.0);   // [A | I], Gauss-Jordan in place
       auto at = [&](long long r, long long c) -> double & { return A[(size_t)r * 2 * n + c]; };
@@ -1425,6 +1729,28 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
         w->cn = (int)n;
       }
     }
+  }
+  if (uni && w->cn > 0 && (rc0 = u_build(m, w, gamb, gens, geew, pinvs))) return rc0;
+  if (uni && !w->u) {   // no dense coarsest inverse, or nothing fits: kernel by kernel
+    if ((rc0 = mg_alloc_field(m, w))) return rc0;
+    uniform_faces64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64);
+    for (int l = 0; l < w->nlev; l++) {
+      MgLevel &L = w->lv[l];
+      if (l == 0) {
+        d2f<<<nb(L.ncell), MGT, 0, m->stream>>>(w->gE64, L.gE, L.ncell);
+        d2f<<<nb(L.ncell), MGT, 0, m->stream>>>(w->gS64, L.gS, L.ncell);
+        d2f<<<nb(L.ncell), MGT, 0, m->stream>>>(w->gB64, L.gB, L.ncell);
+      } else {
+        const MgLevel &F = w->lv[l - 1];
+        mg_coarsen<<<nb(L.ncell), MGT, 0, m->stream>>>(F.gE, F.gS, F.gB, L.gE, L.gS, L.gB, nl, L.nr, L.nc);
+      }
+      mg_diag<<<nb(L.ncell), MGT, 0, m->stream>>>(dev_level(m, L, l), L.diag);
+    }
+    HSB_CUDA(cudaGetLastError());
+  }
+  if (!uni) {
+    u_free(w->u);
+    w->u = nullptr;
   }
   // the coarse levels that fuse into one single-CTA kernel: from the first
   // level of at most MG_FUSE_PLANE columns whose levels down to the coarsest
@@ -1579,14 +1905,32 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   // one refinement pass: r = b - G T (FP64), `inner` PCG iterations on
   // G e = r (FP32), T += e, |e|_2^2 to the host; the same kernel sequence
   // every time, so it is captured once as a CUDA graph and replayed
+  auto residual = [&]() {
+    if (w->u)
+      mgu_residual<<<std::min(nb(m->ncell), 1184u) + 1, MGT, 0, m->stream>>>(w->u->L64, w->d_ps, ge_p, link64, gamb_p, T, w->b64, w->rr,
+                                                            maxbits);
+  };
+  int urc = HSB_OK, pass_iters = 1;
   auto head = [&]() {
     cudaMemsetAsync(maxbits, 0, sizeof(unsigned long long), m->stream);
+    if (w->u) {
+      residual();
+      return;
+    }
     fine_residual64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64, gambL, w->gEdgeNS64,
                                                          w->gEdgeEW64, T, w->b64, w->r64, w->rr, maxbits);
     pack_residual64<<<1, 384, 0, m->stream>>>(S, w->d_ps, ge_p, link64, gamb_p, T, w->b64, w->r64, w->rr, maxbits);
     mg_zero<<<nb(n0), MGT, 0, m->stream>>>(w->e, n0);
   };
   auto iteration = [&](int it) {
+    if (w->u) {
+      // a model within mgu_small: the pass is one launch, made in place of its
+      // first iteration
+      if (w->u->pcg && it > 0) return;
+      const int r = u_iter(m, w, it, pass_iters);
+      if (r) urc = r;
+      return;
+    }
     vcycle(m, w, 0, w->z, w->rr);
     dot(m, w, w->rr, w->z, n0, sc + 2, sc);   // rz (sc[2]); its previous value to sc[0]
     pcg_update_p<<<nb(n0), MGT, 0, m->stream>>>(w->p, w->z, sc, n0, it == 0);
@@ -1597,7 +1941,7 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   auto tail = [&]() {
     // the max norm of this correction (K) decides convergence
     cudaMemsetAsync(sc + 3, 0, sizeof(double), m->stream);
-    add_correction<<<nb(n0), MGT, 0, m->stream>>>(T, w->e, n0, (unsigned long long *)(sc + 3));
+    add_correction<<<std::min(nb(n0), 1184u), MGT, 0, m->stream>>>(T, w->e, n0, (unsigned long long *)(sc + 3));
     cudaMemcpyAsync(w->h_red, sc, sizeof(double) * 5, cudaMemcpyDeviceToHost, m->stream);
   };
   auto capture = [&](auto &&fn, cudaGraphExec_t *out, const char *what) -> int {
@@ -1609,6 +1953,11 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
     HSB_CUDA(cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
     fn();
     const cudaError_t ce = cudaStreamEndCapture(m->stream, &g);
+    if (urc) {
+      if (ce == cudaSuccess && g) cudaGraphDestroy(g);
+      cudaGetLastError();
+      return urc;
+    }
     if (ce != cudaSuccess) return cuda_check(ce, what);
     const cudaError_t ie = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
@@ -1627,12 +1976,14 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   if (!pieces && (!w->pass_exec || w->pass_T != T || w->pass_version != m->coef_version)) {
     if ((rc = capture([&]() {
                         head();
+                        pass_iters = inner;
                         for (int it = 0; it < inner; it++) iteration(it);
                         tail();
                       },
                       &w->pass_exec, "capturing the multigrid refinement pass")) ||
         (rc = capture([&]() {
                         head();
+                        pass_iters = inner_next;
                         for (int it = 0; it < inner_next; it++) iteration(it);
                         tail();
                       },
@@ -1700,9 +2051,13 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   }
   // final FP64 residual for the record
   HSB_CUDA(cudaMemsetAsync(maxbits, 0, sizeof(unsigned long long), m->stream));
-  fine_residual64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64, gambL, w->gEdgeNS64,
-                                                       w->gEdgeEW64, T, w->b64, w->r64, w->rr, maxbits);
-  pack_residual64<<<1, 384, 0, m->stream>>>(S, w->d_ps, ge_p, link64, gamb_p, T, w->b64, w->r64, w->rr, maxbits);
+  if (w->u) {
+    residual();
+  } else {
+    fine_residual64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64, gambL, w->gEdgeNS64,
+                                                         w->gEdgeEW64, T, w->b64, w->r64, w->rr, maxbits);
+    pack_residual64<<<1, 384, 0, m->stream>>>(S, w->d_ps, ge_p, link64, gamb_p, T, w->b64, w->r64, w->rr, maxbits);
+  }
   HSB_CUDA(cudaMemcpyAsync(w->h_red, sc, sizeof(double) * 5, cudaMemcpyDeviceToHost, m->stream));
   HSB_CUDA(cudaStreamSynchronize(m->stream));
   {

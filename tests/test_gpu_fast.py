@@ -266,3 +266,26 @@ def test_paired_passes_shapes(workdir, rows, cols, dt):
     assert np.array_equal(n.grid("trans"), m.grid("trans")) and np.array_equal(tn, t)
     for x in (m, n, q):
         x.close()
+
+
+@pytest.mark.parametrize("rows,cols,layers", [(4, 4, 1), (8, 32, 3), (16, 16, 2), (16, 128, 1), (128, 16, 10), (64, 32, 4),
+                                              (128, 128, 1), (256, 128, 1), (32, 256, 2)])
+def test_mg_steady_shapes(workdir, rows, cols, layers):
+    """The per-layer multigrid at the edges of its parts: one level only, levels
+    one CTA of the cluster takes alone, strips of one and of many rows, whole
+    passes in the cluster and tiles above it.  Against the FP64 sparse direct
+    solution; the solver's tolerance of 1e-8 K leaves an error below it, the
+    direct solution's own is its backward error times the system's condition
+    (1e-16 x 1e7 of 400 K): bar 1e-6 K."""
+    rng = np.random.default_rng([rows, cols, layers])
+    sc = W.scenario_random_chip(workdir, rng, "mg", side=16, chip_layers=layers, steps=1)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    m, o = hm.from_scenario(sc), OracleModel(sc)
+    m.set_solver(FORM_FAST, steady_tol=1e-8)
+    p = m.power_vector(sc.block_power[0] * 0.1)
+    s = m.vector()
+    for _ in range(2):        # the second from the captured passes
+        m.steady(p.copy(), s)
+    g, _ = o.steady_direct(p)
+    assert np.max(np.abs(m.grid("steady") - g)) <= 1e-6
+    m.close()
