@@ -7,6 +7,9 @@ Steady: FP32 multigrid-preconditioned CG inside FP64 iterative refinement;
 compared with the converged FP64 solution of the same system by sparse
 direct LU, bar max |dT| <= 0.01 K (the solver converges far below it).
 """
+import glob
+import os
+
 import numpy as np
 import pytest
 
@@ -266,6 +269,42 @@ def test_paired_passes_shapes(workdir, rows, cols, dt):
     assert np.array_equal(n.grid("trans"), m.grid("trans")) and np.array_equal(tn, t)
     for x in (m, n, q):
         x.close()
+
+
+def _narrow(workdir, by):
+    """Scale the x extents of every floorplan in the directory."""
+    for f in glob.glob(os.path.join(workdir, "*.flp")):
+        rows = [l.split() for l in open(f) if l.strip() and not l.startswith("#")]
+        with open(f, "w") as o:
+            for r in rows:
+                o.write("%s\t%.9e\t%s\t%.9e\t%s\n" % (r[0], float(r[1]) * by, r[2], float(r[3]) * by, r[4]))
+
+
+@pytest.mark.parametrize("rows,cols,layers", [(4, 4, 1), (8, 32, 3), (16, 16, 8), (32, 64, 4), (256, 32, 1), (512, 16, 6),
+                                              (2048, 8, 6)])
+def test_bicgstab_plane_shapes(workdir, rows, cols, layers):
+    """The plane solver at the edges of its parts: planes that are one dense
+    block, few and many reduction steps, an odd number of layers, factors read
+    from global memory (8 layers of 512 rows) and vectors kept there as well
+    (2048 rows; on the narrow grids the die is narrowed to cells of 4:1).  Against the FP64 sparse direct solution; the solver's
+    tolerance of 1e-8 K leaves an error below it, the direct solution's own is
+    its backward error times the system's condition (1e-16 x 1e7 of 400 K): bar
+    1e-6 K."""
+    from hotspot_b200 import STEADY_BICGSTAB
+    rng = np.random.default_rng([rows, cols, layers])
+    sc = W.scenario_random_chip(workdir, rng, "bc", side=16, chip_layers=layers, steps=1)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    if rows > 8 * cols:
+        _narrow(workdir, 4 * cols / rows)
+    m, o = hm.from_scenario(sc), OracleModel(sc)
+    m.set_solver(FORM_FAST, STEADY_BICGSTAB, steady_tol=1e-8)
+    p = m.power_vector(sc.block_power[0] * 0.1)
+    s = m.vector()
+    for _ in range(2):        # the second from the captured passes
+        m.steady(p.copy(), s)
+    g, _ = o.steady_direct(p)
+    assert np.max(np.abs(m.grid("steady") - g)) <= 1e-6
+    m.close()
 
 
 @pytest.mark.parametrize("rows,cols,layers", [(4, 4, 1), (8, 32, 3), (16, 16, 2), (16, 128, 1), (128, 16, 10), (64, 32, 4),
