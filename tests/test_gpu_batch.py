@@ -128,6 +128,28 @@ def test_batch_autotuner(workdir):
     assert max(errs) <= TOL, errs
 
 
+@pytest.mark.parametrize("ctas", [1, 2, 7, 0])
+def test_batch_cta_groups(workdir, ctas):
+    """The CTA groups of the shortest launch: every chip on one CTA, one group
+    beside packed chips, more tiles than CTAs and more CTAs than needed.  The
+    sums do not depend on the groups: the single-model form within 1e-9 K."""
+    scs = _chips(workdir, [("stack3d", 128), ("chip2d", 32), ("random", 64), ("chip2d", 64)])
+    single, batched = _models(scs)
+    bt = Batch(batched)
+    bt.set_ctas(ctas)
+    for c, a in enumerate(single):
+        a.set_tile(*bt.tile(c))
+        for k in (1, 2):
+            a.compute_temp(a.power_vector(scs[c].block_power[k]), None, scs[c].dt)
+    bt.trace([[b.power_vector(sc.block_power[k]) for sc, b in zip(scs, batched)] for k in (1, 2)], scs[0].dt)
+    errs = [float(np.max(np.abs(a.grid("trans") - b.grid("trans")))) for a, b in zip(single, batched)]
+    assert bt.info()["grid"] >= 1 and (ctas == 0 or bt.info()["grid"] <= ctas)
+    bt.close()
+    for m in single + batched:
+        m.close()
+    assert max(errs) <= TOL, errs
+
+
 def test_batch_subset_launches(workdir):
     """Launches over a subset of the models, a few intervals each (the ticks of
     the serving batch engine): the listed chips match the single-model form
