@@ -754,7 +754,9 @@ def run_ours(args):
     # the kernel's own events; if the library could not time it, the whole interval
     kernel_timed = ker_ms > 0
     achieved = alg_bytes_launch / (((ker_ms if kernel_timed else dev_ms) / K) / 1e3) / 1e9
-    kname = {"passes": "rk4_krylov_kernel", "blocked": "rk4_tb_kernel"}.get(head_kernel, head_kernel)
+    # the pass-by-pass form keeps grids that fit the SMs' shared memory there
+    passes = "rk4_pair_kernel" if args.grid <= 256 else "rk4_krylov_kernel"
+    kname = {"passes": passes, "blocked": "rk4_tb_kernel"}.get(head_kernel, head_kernel)
     traffic = profiled_traffic(f"{kname}_stack256.md")
     line = {
         "metric": METRIC, "value": value, "unit": "cell-steps/s", "n_gpus": ws, "steps": K,

@@ -26,10 +26,10 @@
 // An iteration at 256x256 is 6 launches where kernel by kernel it was 42, most
 // of them a few microseconds of launch and drain around little work.  Steady
 // states on B200, before and after: 64x64x4 1879 -> 729 us, 256x256x6 3413 ->
-// 1578 us, 1024x1024x4 11047 -> 4642 us.  What is left: mgu_small is bound by
+// 1578 us, 1024x1024x5 11047 -> 4642 us.  What is left: mgu_small is bound by
 // its cluster barriers (about 1000 cycles each; 70 us an iteration from 128x128
-// down), the tiled kernels at 1024x1024 by memory (apply 50 us, post 49, down
-// 28, pre 20, step 16).  The residual and correction kernels of mg_steady.cu
+// down); the tiled kernels at 1024x1024 (apply 50 us, post 49, down 28, pre 20,
+// step 16) run at up to a quarter of the copy rate.  The residual and correction kernels of mg_steady.cu
 // were bound by one atomic per warp on a single word; they take one per CTA.
 #pragma once
 #include <cooperative_groups.h>

@@ -698,9 +698,10 @@ static int tb_prepare_single(hsb_dev_model *m, FastWork *w) {
 // temporally blocked kernel: its working set (two FP64 states, the Krylov
 // vectors of the pass-by-pass form) no longer fits L2, and it reads the state
 // once per attempt instead of streaming a vector per pass.  Below, the
-// pass-by-pass kernel: its passes run from L2 and an attempt recomputes no
-// halo (on a B200 it is 1.5x faster on a 256x256x6 stack, 1.2x on a 64x64x3
-// chip).  The choice depends on the model's shape only, so a model's results
+// pass-by-pass kernels, whose attempts recompute no halo: where the SMs can
+// hold the grid the one that keeps its vectors in shared memory (rk4_pair.cu,
+// an interval of 256x256x6 in 188 us), else the one that runs from L2 (249 us
+// there, 1.5x faster than the blocked kernel; 1.2x on a 64x64x3 chip).  The choice depends on the model's shape only, so a model's results
 // do not depend on when or beside what it runs.
 #define TB_MIN_CELLS (1LL << 21)
 int kry_prepare(hsb_dev_model *m, FastWork *w) {

@@ -47,7 +47,7 @@ extern "C" {
                                    within 1e-6 K of the FP64 replay; steady as HSB_FORM_PARITY */
 #define HSB_FORM_FAST_BLOCKED 5 /* the fast transient on the temporally blocked kernel
                                    whatever the model's size (HSB_FORM_FAST takes it from
-                                   2^21 cells up, the pass-by-pass kernel below) */
+                                   2^21 cells up, a pass-by-pass kernel below) */
 
 /* steady methods */
 #define HSB_STEADY_AUTO       0  /* GS replay for FORM_PARITY; MG-PCG (or BiCGStab with advection) for FORM_FAST */
