@@ -972,11 +972,16 @@ __global__ void dot_one(const float *__restrict__ a, const float *__restrict__ b
   }
 }
 
+// a step length of the conjugate gradients.  A residual that is zero to begin
+// with (no power and everything at ambient) has (r, z) = (p, q) = 0: no step.
+// Anything else that does not divide reaches the correction, whose norm then
+// reports it.
+__device__ __forceinline__ float mg_ratio(double a, double b) { return a == 0.0 ? 0.f : (float)(a / b); }
+
 // x += alpha p; r -= alpha q   with alpha = rz / pq  (sc[2] rz, sc[1] pq)
 __global__ void pcg_update_xr(float *__restrict__ x, float *__restrict__ r, const float *__restrict__ p,
                               const float *__restrict__ q, const double *__restrict__ sc, long long n) {
-  const double alpha = sc[2] / sc[1];
-  const float a = (float)alpha;
+  const float a = mg_ratio(sc[2], sc[1]);
   long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k < n) {
     x[k] += a * p[k];
@@ -994,12 +999,13 @@ __global__ void pcg_update_p(float *__restrict__ p, const float *__restrict__ z,
     p[k] = z[k];
     return;
   }
-  const float beta = (float)(sc[2] / sc[0]);
+  const float beta = mg_ratio(sc[2], sc[0]);
   p[k] = z[k] + beta * p[k];
 }
 
-// T += e; the max |e| (K) into *emax_bits (zeroed by the caller), one atomic
-// per CTA (one per warp was most of the time on large grids)
+// T += e; the max |e| (K) into *emax_bits (zeroed by the caller), infinite if
+// an entry is not a number (which a maximum would drop); one atomic per CTA
+// (one per warp was most of the time on large grids)
 __global__ void __launch_bounds__(MGT) add_correction(double *__restrict__ T, const float *__restrict__ e, long long n,
                                                       unsigned long long *emax_bits) {
   __shared__ double wm[MGT / 32];
@@ -1007,7 +1013,7 @@ __global__ void __launch_bounds__(MGT) add_correction(double *__restrict__ T, co
   for (long long k = (long long)blockIdx.x * MGT + threadIdx.x; k < n; k += (long long)gridDim.x * MGT) {
     const double d = (double)e[k];
     T[k] += d;
-    a = fmax(a, fabs(d));
+    a = fmax(a, d == d ? fabs(d) : INFINITY);
   }
   for (int o = 16; o > 0; o >>= 1) a = fmax(a, __shfl_down_sync(0xffffffffu, a, o));
   if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = a;
@@ -2035,6 +2041,7 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
     }
     st->refinements += 1;
     st->cycles += n_it;
+    if (!std::isfinite(emax)) return set_error(HSB_E_NOCONV, "multigrid steady solve broke down (a correction is not finite)");
     if (emax < tol) {
       converged = true;
       break;

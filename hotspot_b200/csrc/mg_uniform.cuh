@@ -869,7 +869,7 @@ __global__ void __launch_bounds__(MGU_ST) mgu_small(const __grid_constant__ USma
       if (rank == 0 && tid < nx) d += (double)rpk[tid] * (double)xp[0][tid];
       const double rz_old = rz;
       rz = all_sum(d, 0);
-      const float beta = it == 0 ? 0.f : (float)(rz / rz_old);
+      const float beta = it == 0 ? 0.f : mg_ratio(rz, rz_old);
       for (int k = tid; k < own; k += MGU_ST) {
 #pragma unroll
         for (int n = 0; n < NL; n++) pv[n * sz + k] = it == 0 ? z[n * sz + k] : z[n * sz + k] + beta * pv[n * sz + k];
@@ -911,7 +911,7 @@ __global__ void __launch_bounds__(MGU_ST) mgu_small(const __grid_constant__ USma
         if (rank == 0) d += (double)v * (double)ppk[tid];
       }
       const double pq = all_sum(d, 1);
-      const float alpha = (float)(rz / pq);
+      const float alpha = mg_ratio(rz, pq);
       for (int k = tid; k < own; k += MGU_ST) {
 #pragma unroll
         for (int n = 0; n < NL; n++) {
@@ -970,7 +970,7 @@ __global__ void __launch_bounds__(MGU_T) mgu_apply(const __grid_constant__ ULev 
   const int which = *(volatile int *)par;
   const float *po = which ? p1 : p0;
   float *pn = which ? p0 : p1;
-  const float beta = first ? 0.f : (float)(sc[2] / sc[0]);
+  const float beta = first ? 0.f : mg_ratio(sc[2], sc[0]);
   auto dir = [&](long long c) { return first ? z[c] : z[c] + beta * po[c]; };
   if (threadIdx.x < nx) xp[threadIdx.x] = dir(ncell + threadIdx.x);
   for (int k = threadIdx.x; k < U_H1 * U_W1; k += MGU_T) {
@@ -1037,7 +1037,7 @@ __global__ void __launch_bounds__(256) mgu_step(float *__restrict__ e, float *__
                                                 const float *p1, const int *par, const float *__restrict__ q,
                                                 const double *__restrict__ sc, long long n, int first) {
   const float *p = *par ? p1 : p0;
-  const float a = (float)(sc[2] / sc[1]);
+  const float a = mg_ratio(sc[2], sc[1]);
   const long long k = 4 * ((long long)blockIdx.x * blockDim.x + threadIdx.x);
   if (k + 3 < n) {
     const float4 P = *(const float4 *)(p + k), Q = *(const float4 *)(q + k);

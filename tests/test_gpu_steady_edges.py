@@ -1,0 +1,53 @@
+"""The fast steady solvers where their iterations have nothing to do, are given
+something they cannot solve, or meet a model that has changed."""
+import numpy as np
+import pytest
+
+from hotspot_b200 import FORM_FAST
+from hotspot_b200 import model as hm
+from hotspot_b200 import workloads as W
+from hotspot_b200._abi import HotspotError
+
+pytestmark = pytest.mark.gpu
+
+# one level; whole passes in the cluster; tiles above it; kernel by kernel
+MG_CASES = [(4, 8, False), (16, 16, False), (256, 128, False), (16, 16, True)]
+
+
+def _chip(workdir, rows, cols, detailed, seed=5):
+    sc = W.scenario_chip2d(workdir, seed=seed, grid=16, steps=1, n_blocks=3)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    sc.detailed_3D = detailed
+    return sc
+
+
+@pytest.mark.parametrize("rows,cols,detailed", MG_CASES)
+def test_mg_steady_without_power(workdir, rows, cols, detailed):
+    """No power: everything is at ambient, where the first residual is zero to
+    the last bit, and the step lengths of the conjugate gradients are 0 / 0."""
+    m = hm.from_scenario(_chip(workdir, rows, cols, detailed))
+    m.set_solver(FORM_FAST)
+    s = m.vector()
+    for _ in range(2):
+        m.steady(m.vector(), s)
+        assert np.array_equal(m.grid("steady"), np.full(m.n_cells + m.n_extra, m.config.ambient))
+        assert np.array_equal(s, m.vector(m.config.ambient))
+    m.close()
+
+
+@pytest.mark.parametrize("rows,cols,detailed", MG_CASES)
+def test_mg_steady_of_a_power_that_is_no_number(workdir, rows, cols, detailed):
+    """An error, not temperatures that are no numbers; the model solves on."""
+    sc = _chip(workdir, rows, cols, detailed)
+    m = hm.from_scenario(sc)
+    m.set_solver(FORM_FAST)
+    p = m.power_vector(sc.block_power[0])
+    s, t = m.vector(), m.vector()
+    m.steady(p.copy(), s)
+    bad = p.copy()
+    bad[np.flatnonzero(p)[0]] = np.nan
+    with pytest.raises(HotspotError, match="not finite"):
+        m.steady(bad, t)
+    m.steady(p.copy(), t)
+    assert np.array_equal(s, t)
+    m.close()
