@@ -1145,7 +1145,8 @@ __global__ void __launch_bounds__(BCT) bc_update_er(float *__restrict__ e, float
   }
 }
 
-// T += e; the max |e| (K) into *emax_bits (zeroed by the caller)
+// T += e; the max |e| (K) into *emax_bits (zeroed by the caller), infinite if
+// an entry is not a number (which a maximum would drop)
 __global__ void bc_add_correction(double *__restrict__ T, const float *__restrict__ e, unsigned n, int nl, int nr,
                                   int nc, unsigned long long *emax_bits) {
   const unsigned k = blockIdx.x * blockDim.x + threadIdx.x, ncell = (unsigned)nl * nr * nc;
@@ -1153,7 +1154,7 @@ __global__ void bc_add_correction(double *__restrict__ T, const float *__restric
   if (k < n) {
     const double d = (double)e[k < ncell ? bc_cell_of(k, nl, nr, nc) : k];
     T[k] += d;
-    a = fabs(d);
+    a = d == d ? fabs(d) : INFINITY;
   }
   bc_block_max(a, emax_bits);
 }
@@ -1624,7 +1625,7 @@ int bicgstab_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
     if (lost) return set_error(HSB_E_CUDA, "BiCGStab plane solve: a copy of the factors did not complete in time");
     st->refinements += 1;
     st->cycles += p ? BC_LAST : BC_INNER;
-    if (!(emax == emax)) return set_error(HSB_E_NOCONV, "BiCGStab steady solve broke down (NaN correction)");
+    if (!std::isfinite(emax)) return set_error(HSB_E_NOCONV, "BiCGStab steady solve broke down (a correction is not finite)");
     if (emax < tol) {
       converged = true;
       break;

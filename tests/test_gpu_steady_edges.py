@@ -35,10 +35,12 @@ def test_mg_steady_without_power(workdir, rows, cols, detailed):
     m.close()
 
 
-@pytest.mark.parametrize("rows,cols,detailed", MG_CASES)
-def test_mg_steady_of_a_power_that_is_no_number(workdir, rows, cols, detailed):
-    """An error, not temperatures that are no numbers; the model solves on."""
-    sc = _chip(workdir, rows, cols, detailed)
+def _uchan(workdir, seed=2, **kw):
+    return W.scenario_microchannel(workdir, seed=seed, **(kw or dict(
+        grid=32, die=2e-3, channel_w=125e-6, channel_h=125e-6, pitch=250e-6, blocks=8)))
+
+
+def _power_that_is_no_number(sc):
     m = hm.from_scenario(sc)
     m.set_solver(FORM_FAST)
     p = m.power_vector(sc.block_power[0])
@@ -51,3 +53,13 @@ def test_mg_steady_of_a_power_that_is_no_number(workdir, rows, cols, detailed):
     m.steady(p.copy(), t)
     assert np.array_equal(s, t)
     m.close()
+
+
+@pytest.mark.parametrize("rows,cols,detailed", MG_CASES)
+def test_mg_steady_of_a_power_that_is_no_number(workdir, rows, cols, detailed):
+    """An error, not temperatures that are no numbers; the model solves on."""
+    _power_that_is_no_number(_chip(workdir, rows, cols, detailed))
+
+
+def test_bicgstab_steady_of_a_power_that_is_no_number(workdir):
+    _power_that_is_no_number(_uchan(workdir))
