@@ -159,7 +159,8 @@ struct BcWork {
   int *status;                 // raised by a plane solve whose factors did not arrive
   unsigned *done;              // CTAs that have finished (kernels whose last CTA goes on)
   cudaGraphExec_t pass_exec[2];   // of BC_INNER and of BC_LAST iterations
-  const double *pass_T;        // the state buffer the graphs were captured for
+  const double *pass_T;        // the state buffer and the coefficients the graphs were captured for
+  int pass_version;            // (package and edge conductances are kernel arguments)
   long long pass_launches[2];
 };
 
@@ -1597,13 +1598,14 @@ int bicgstab_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   long long launches = 0;
   bc_fill<<<bnb(n0), BCT, 0, m->stream>>>(T, m->ambient, n0);
   HSB_CUDA(cudaGetLastError());
-  if (w->pass_T != T) {
+  if (w->pass_T != T || w->pass_version != m->coef_version) {
     for (auto &g : w->pass_exec)
       if (g) {
         cudaGraphExecDestroy(g);
         g = nullptr;
       }
     w->pass_T = T;
+    w->pass_version = m->coef_version;
   }
   // stopping as in the multigrid solver: the last correction below tol, or
   // passes contracting so fast (rho = |e_k| / |e_k-1| < 0.1) that the next

@@ -3,7 +3,7 @@ something they cannot solve, or meet a model that has changed."""
 import numpy as np
 import pytest
 
-from hotspot_b200 import FORM_FAST
+from hotspot_b200 import FORM_FAST, STEADY_AUTO, STEADY_BICGSTAB
 from hotspot_b200 import model as hm
 from hotspot_b200 import workloads as W
 from hotspot_b200._abi import HotspotError
@@ -63,3 +63,29 @@ def test_mg_steady_of_a_power_that_is_no_number(workdir, rows, cols, detailed):
 
 def test_bicgstab_steady_of_a_power_that_is_no_number(workdir):
     _power_that_is_no_number(_uchan(workdir))
+
+
+@pytest.mark.parametrize("what,method", [("chip", STEADY_AUTO), ("chip", STEADY_BICGSTAB), ("uchan", STEADY_AUTO)])
+def test_steady_after_the_package_changed(workdir, what, method):
+    """A model that has solved once and is given another spreader and sink (the
+    package's and the edges' conductances change) solves as a fresh model with
+    them does: the same passes and the same bits."""
+    sc = _uchan(workdir) if what == "uchan" else _chip(workdir, 32, 32, False)
+    new = {"s_spreader": "0.05", "s_sink": "0.09"}
+    m = hm.from_scenario(sc)
+    sc.config.update(new)
+    f = hm.from_scenario(sc)
+    p, s, t = m.power_vector(sc.block_power[0]), m.vector(), m.vector()
+    for x in (m, f):
+        x.set_solver(FORM_FAST, method)
+    m.steady(p.copy(), s)
+    cfg = m.ptr.contents.config
+    cfg.s_spreader, cfg.s_sink = float(new["s_spreader"]), float(new["s_sink"])
+    hm.populate_R_model(m, m._flp)
+    m.steady(p.copy(), s)
+    f.steady(p.copy(), t)
+    a, b = m.stats(), f.stats()
+    assert (a["refinements"], a["cycles"]) == (b["refinements"], b["cycles"])
+    assert np.array_equal(m.grid("steady"), f.grid("steady")) and np.array_equal(s, t)
+    m.close()
+    f.close()
