@@ -636,25 +636,29 @@ __global__ void __launch_bounds__(MGU_ST) mgu_small(const __grid_constant__ USma
   auto edge_parts = [&](int l) {
     u_edge_parts_strip(sL[l], sm + off[l], u_strip(sL[l].nr, sL[l].nc), rank, nullptr, part);
   };
-  // the edge sums from every strip's share into es, in each CTA
   auto solo = [&](int l) { return sL[l].nr * sL[l].nc <= MGU_SOLO; };
   auto sync = [&](int l) {   // between the phases of level l
     if (solo(l)) __syncthreads();
     else cl.sync();
   };
-  auto gather = [&](int l) {
+  // the edge sums from every strip's share into es, in each CTA (behind a cluster barrier)
+  auto gather_all = [&]() {
     const int ne = sL[0].ne, lane = tid & 15;
-    if (solo(l)) {
-      if (tid < ne) es[tid] = part[tid];
-      __syncthreads();
-      return;
-    }
     for (int e0 = 0; e0 < ne; e0 += MGU_ST / 16) {
       const int e = e0 + (tid >> 4);
       float s = e < ne ? *cl.map_shared_rank(&part[e], lane) : 0.f;
       for (int o = 8; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o, 16);
       if (e < ne && lane == 0) es[e] = s;
     }
+    __syncthreads();
+  };
+  // ... of a level that one CTA takes alone: there only
+  auto gather = [&](int l) {
+    if (!solo(l)) {
+      gather_all();
+      return;
+    }
+    if (tid < sL[0].ne) es[tid] = part[tid];
     __syncthreads();
   };
   // the package nodes of level l, in each CTA
@@ -789,7 +793,7 @@ __global__ void __launch_bounds__(MGU_ST) mgu_small(const __grid_constant__ USma
         v = cl.map_shared_rank(sm + off[last] + NL * sz, o)[n * sz + (i - o * rp) * nc + k - i * nc];
       } else {
         const int k = q - NL * plane;
-        v = last == 0 && k < nx ? S.f[(long long)NL * plane + k] : 0.f;
+        v = last == 0 && k < nx ? rpk[k] : 0.f;   // (a single level: the residual as it is now)
       }
       coarse[q] = v;
     }
@@ -878,7 +882,7 @@ __global__ void __launch_bounds__(MGU_ST) mgu_small(const __grid_constant__ USma
       __syncthreads();
       u_edge_parts_strip(L, pv, rp, rank, ppk, part);
       cl.sync();
-      gather(0);
+      gather_all();   // every CTA keeps the package's residual: with a single level its exact solve takes it
       d = 0.0;
       for (int k = tid; k < own; k += MGU_ST) {
         const int kr = k / nc, i = rank * rp + kr, j = k - kr * nc;

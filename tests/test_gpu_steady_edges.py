@@ -89,3 +89,20 @@ def test_steady_after_the_package_changed(workdir, what, method):
     assert np.array_equal(m.grid("steady"), f.grid("steady")) and np.array_equal(s, t)
     m.close()
     f.close()
+
+
+@pytest.mark.parametrize("rows,cols,tol", [(4, 16, 1e-9), (1, 16, 1e-9), (4, 8, 1e-10), (8, 4, 1e-10)])
+def test_mg_single_level_refinements(workdir, rows, cols, tol):
+    """Grids that are one level of the multigrid: its exact solve takes the
+    residual of each iteration, package nodes included, so a per-layer model
+    (whole passes in the cluster) needs no more passes than the same model with
+    per-cell coefficients (kernel by kernel)."""
+    passes = []
+    for detailed in (False, True):
+        sc = _chip(workdir, rows, cols, detailed)
+        m = hm.from_scenario(sc)
+        m.set_solver(FORM_FAST, steady_tol=tol)
+        m.steady(m.power_vector(sc.block_power[0]), m.vector())
+        passes.append(m.stats()["refinements"])
+        m.close()
+    assert passes[0] <= passes[1]
