@@ -19,6 +19,7 @@ int set_error(int code, const std::string &msg) {
 }
 
 int cuda_check(cudaError_t e, const char *what) {
+  cudaGetLastError();   // reported here: must not surface again in a later call's check
   return set_error(e == cudaErrorMemoryAllocation ? HSB_E_NOMEM : HSB_E_CUDA,
                    std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -1141,20 +1141,24 @@ struct MgUniform {
   bool pcg;                    // the whole pass in mgu_small
 };
 
+static void u_small_config(hsb_dev_model *m, const MgUniform &u, cudaLaunchConfig_t *cfg, cudaLaunchAttribute *attr) {
+  memset(cfg, 0, sizeof(*cfg));
+  cfg->gridDim = dim3(MGU_CL);
+  cfg->blockDim = dim3(MGU_ST);
+  cfg->dynamicSmemBytes = u.small_smem;
+  cfg->stream = m->stream;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = MGU_CL;
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
+}
+
 template <int NL, bool PCG>
 static int u_launch_small(hsb_dev_model *m, const MgUniform &u, const USmall &S) {
   cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(MGU_CL);
-  cfg.blockDim = dim3(MGU_ST);
-  cfg.dynamicSmemBytes = u.small_smem;
-  cfg.stream = m->stream;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = MGU_CL;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  u_small_config(m, u, &cfg, attr);
   HSB_CUDA(cudaLaunchKernelEx(&cfg, mgu_small<NL, PCG>, S));
   return HSB_OK;
 }
@@ -1231,13 +1235,24 @@ static int u_iter(hsb_dev_model *m, MgWork *w, int it, int n_it) {
   return rc;
 }
 
-static int u_small_setup(int nl, size_t smem, bool pcg) {
+// mgu_small's attributes; *fits: the device can place its cluster (16 CTAs are
+// more than the portable 8, and each takes most of an SM's shared memory)
+static int u_small_setup(hsb_dev_model *m, const MgUniform &u, bool *fits) {
   const void *fn = nullptr;
-#define U_CALL(N) fn = pcg ? (const void *)mgu_small<N, true> : (const void *)mgu_small<N, false>
-  U_DISPATCH(nl, U_CALL)
+#define U_CALL(N) fn = u.pcg ? (const void *)mgu_small<N, true> : (const void *)mgu_small<N, false>
+  U_DISPATCH(m->nl, U_CALL)
 #undef U_CALL
-  HSB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  return raise_smem_limit(fn, smem);
+  *fits = false;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[1];
+  u_small_config(m, u, &cfg, attr);
+  int clusters = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      raise_smem_limit(fn, u.small_smem) != HSB_OK || cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess)
+    cudaGetLastError();   // refused: the solve goes kernel by kernel
+  else
+    *fits = clusters > 0;
+  return HSB_OK;
 }
 
 static void u_free(MgUniform *u) {
@@ -1260,8 +1275,7 @@ static cudaError_t mg_alloc(Tp **p, size_t bytes, cudaStream_t s) {
   return e;
 }
 
-static int mg_setup(hsb_dev_model *m, MgWork **out) {
-  MgWork *w = new MgWork();
+static int mg_setup(hsb_dev_model *m, MgWork *w) {
   w->coef_version = -1;
   const int nl = m->nl, nx = m->nx;
   // levels: halve while both sides are even and >= 4 (keep >= 2x2 columns)
@@ -1303,23 +1317,24 @@ static int mg_setup(hsb_dev_model *m, MgWork **out) {
   if (w->lv[0].plane >= (1LL << 31) - MGT) return set_error(HSB_E_ARG, "multigrid: more than 2^31 columns per layer");
 
   HSB_CUDA(cudaMallocHost(&w->h_red, sizeof(double) * 8));
-  *out = w;
   return HSB_OK;
 }
 
 // the per-cell operators' arrays, for models that need them
 static int mg_alloc_field(hsb_dev_model *m, MgWork *w) {
   if (w->field) return HSB_OK;
+  // (those that an earlier call got before it failed stay)
+  auto get = [&](auto **p, size_t bytes) { return *p ? cudaSuccess : mg_alloc(p, bytes, m->stream); };
   for (auto &L : w->lv) {
-    HSB_CUDA(mg_alloc(&L.gE, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.gS, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.gB, sizeof(float) * L.ncell, m->stream));
-    HSB_CUDA(mg_alloc(&L.diag, sizeof(float) * L.ncell, m->stream));
+    HSB_CUDA(get(&L.gE, sizeof(float) * L.ncell));
+    HSB_CUDA(get(&L.gS, sizeof(float) * L.ncell));
+    HSB_CUDA(get(&L.gB, sizeof(float) * L.ncell));
+    HSB_CUDA(get(&L.diag, sizeof(float) * L.ncell));
   }
-  HSB_CUDA(mg_alloc(&w->gE64, sizeof(double) * m->ncell, m->stream));
-  HSB_CUDA(mg_alloc(&w->gS64, sizeof(double) * m->ncell, m->stream));
-  HSB_CUDA(mg_alloc(&w->gB64, sizeof(double) * m->ncell, m->stream));
-  HSB_CUDA(mg_alloc(&w->r64, sizeof(double) * w->lv[0].n, m->stream));
+  HSB_CUDA(get(&w->gE64, sizeof(double) * m->ncell));
+  HSB_CUDA(get(&w->gS64, sizeof(double) * m->ncell));
+  HSB_CUDA(get(&w->gB64, sizeof(double) * m->ncell));
+  HSB_CUDA(get(&w->r64, sizeof(double) * w->lv[0].n));
   w->field = true;
   return HSB_OK;
 }
@@ -1397,47 +1412,68 @@ static float u_diag(const ULev &L, int n, bool i0, bool i1, bool j0, bool j1) {
   return d;
 }
 
-// the per-layer models' tables and buffers; w->u stays null where the small
-// levels do not fit
+// the per-layer models' buffers.  *out stays null where the small levels do not
+// fit mgu_small or the device cannot place its cluster; on an error nothing is
+// left behind either, so that the next solve starts over.
+static int u_create(hsb_dev_model *m, const MgWork *w, const double *gamb, const double *gens, const double *geew,
+                    MgUniform **out) {
+  const int nl = m->nl;
+  // the finest level from which on everything fits
+  int c = 0;
+  size_t smem = 0;
+  bool pcg = false;
+  for (; c < w->nlev; c++) {
+    const MgLevel &L = w->lv[c];
+    if (L.plane > MGU_SMALL || w->nlev - c > MGU_SLEV || u_strip(L.nr, L.nc) * (L.nc / 2) > MGU_ST) continue;
+    USmall S;
+    memset(&S, 0, sizeof(S));
+    S.nlev = w->nlev - c;
+    S.cn = w->cn;
+    for (int k = 0; k < S.nlev; k++) S.L[k] = u_level(m, w, c + k, gamb, gens, geew);
+    pcg = c == 0;
+    smem = sizeof(float) * u_small_floats(S, nl, m->nx, pcg);
+    if (smem <= 200 * 1024) break;
+  }
+  if (c == w->nlev || w->nlev > 24) return HSB_OK;
+  MgUniform *u = new MgUniform();
+  memset(u, 0, sizeof(*u));
+  u->nlev = w->nlev;
+  u->small = c;
+  u->pcg = pcg;
+  u->small_smem = smem;
+  const int seg_c = (m->nc + MGU_TC - 1) / MGU_TC, seg_r = (m->nr + MGU_TR - 1) / MGU_TR;
+  const size_t blocks = (size_t)seg_c * seg_r;
+  u->seg = std::max(seg_c, seg_r);
+  bool fits = false;
+  auto build = [&]() -> int {
+    const int rc = u_small_setup(m, *u, &fits);
+    if (rc || !fits) return rc;
+    HSB_CUDA(mg_alloc(&u->tab, sizeof(float) * w->nlev * u_tab_floats(nl, m->nx), m->stream));
+    HSB_CUDA(mg_alloc(&u->epart, sizeof(float) * 20 * (u->seg + w->nlev), m->stream));
+    HSB_CUDA(mg_alloc(&u->part, sizeof(double) * blocks, m->stream));
+    HSB_CUDA(mg_alloc(&u->ticket, 64, m->stream));
+    HSB_CUDA(mg_alloc(&u->p2, sizeof(float) * w->lv[0].n, m->stream));
+    return HSB_OK;
+  };
+  const int rc = build();
+  if (rc || !fits) {
+    u_free(u);
+    return rc;
+  }
+  u->esum = u->epart + 20 * u->seg;
+  u->par = (int *)(u->ticket + 8);
+  *out = u;
+  return HSB_OK;
+}
+
+// the tables of the model's present conductances; w->u stays null where u_create
+// makes nothing
 static int u_build(hsb_dev_model *m, MgWork *w, const double *gamb, const double *gens, const double *geew,
                    const std::vector<float> &pinv) {
   const int nl = m->nl;
   if (!w->u) {
-    // the finest level from which on everything fits mgu_small
-    int c = 0;
-    size_t smem = 0;
-    bool pcg = false;
-    for (; c < w->nlev; c++) {
-      const MgLevel &L = w->lv[c];
-      if (L.plane > MGU_SMALL || w->nlev - c > MGU_SLEV || u_strip(L.nr, L.nc) * (L.nc / 2) > MGU_ST) continue;
-      USmall S;
-      memset(&S, 0, sizeof(S));
-      S.nlev = w->nlev - c;
-      S.cn = w->cn;
-      for (int k = 0; k < S.nlev; k++) S.L[k] = u_level(m, w, c + k, gamb, gens, geew);
-      pcg = c == 0;
-      smem = sizeof(float) * u_small_floats(S, nl, m->nx, pcg);
-      if (smem <= 200 * 1024) break;
-    }
-    if (c == w->nlev || w->nlev > 24) return HSB_OK;
-    MgUniform *u = new MgUniform();
-    memset(u, 0, sizeof(*u));
-    u->nlev = w->nlev;
-    u->small = c;
-    u->pcg = pcg;
-    u->small_smem = smem;
-    const size_t blocks = (size_t)((m->nc + MGU_TC - 1) / MGU_TC) * ((m->nr + MGU_TR - 1) / MGU_TR);
-    w->u = u;
-    u->seg = std::max((m->nc + MGU_TC - 1) / MGU_TC, (m->nr + MGU_TR - 1) / MGU_TR);
-    HSB_CUDA(mg_alloc(&u->tab, sizeof(float) * w->nlev * u_tab_floats(nl, m->nx), m->stream));
-    HSB_CUDA(mg_alloc(&u->epart, sizeof(float) * 20 * (u->seg + w->nlev), m->stream));
-    u->esum = u->epart + 20 * u->seg;
-    HSB_CUDA(mg_alloc(&u->part, sizeof(double) * blocks, m->stream));
-    HSB_CUDA(mg_alloc(&u->ticket, 64, m->stream));
-    HSB_CUDA(mg_alloc(&u->p2, sizeof(float) * w->lv[0].n, m->stream));
-    u->par = (int *)(u->ticket + 8);
-    int rc;
-    if ((rc = u_small_setup(nl, u->small_smem, u->pcg))) return rc;
+    const int rc = u_create(m, w, gamb, gens, geew, &w->u);
+    if (rc || !w->u) return rc;
   }
   MgUniform &u = *w->u;
   const size_t tf = u_tab_floats(nl, m->nx);
@@ -1885,7 +1921,11 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   MgWork *w = (MgWork *)m->mg;
   int rc;
   if (!w) {
-    if ((rc = mg_setup(m, &w))) return rc;
+    w = new MgWork();
+    if ((rc = mg_setup(m, w))) {
+      free_mg(w);
+      return rc;
+    }
     m->mg = w;
     m->mg_free = free_mg;
   }

@@ -106,3 +106,49 @@ def test_mg_single_level_refinements(workdir, rows, cols, tol):
         passes.append(m.stats()["refinements"])
         m.close()
     assert passes[0] <= passes[1]
+
+
+def test_mg_out_of_memory_then_again(workdir):
+    """A steady solve that runs out of device memory while it sets its workspace
+    up (the last of its vectors does not fit) reports that, and the model solves
+    once there is room."""
+    import torch
+
+    sc = _chip(workdir, 1024, 1024, False)
+
+    def model():
+        m = hm.from_scenario(sc)
+        m.set_solver(FORM_FAST)
+        return m, m.power_vector(sc.block_power[0])
+
+    def free():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    for _ in range(2):        # the first loads the kernels, the second is measured
+        m, p = model()
+        want = m.vector()
+        before = free()
+        m.steady(p.copy(), want)
+        workspace = before - free()
+        m.close()
+    vec = 4 * 4 * 1024 * 1024
+    assert workspace > 10 * vec
+    raised, base = 0, free()
+    for short in (4 << 20, vec // 2, vec, 6 * vec):
+        m, p = model()
+        hog = torch.empty(free() - (workspace - short), dtype=torch.uint8, device="cuda")
+        try:
+            m.steady(p.copy(), m.vector())
+        except HotspotError as e:
+            assert "memory" in str(e)
+            raised += 1
+        del hog
+        free()
+        s = m.vector()
+        m.steady(p.copy(), s)
+        assert np.array_equal(s, want)
+        m.close()
+        assert free() > base - vec
+    assert raised >= 2
