@@ -1772,7 +1772,12 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
       }
     }
   }
-  if (uni && w->cn > 0 && (rc0 = u_build(m, w, gamb, gens, geew, pinvs))) return rc0;
+  if (!uni || w->cn == 0) {   // also where an earlier build's coarsest operator had an inverse and this one has none
+    u_free(w->u);
+    w->u = nullptr;
+  } else if ((rc0 = u_build(m, w, gamb, gens, geew, pinvs))) {
+    return rc0;
+  }
   if (uni && !w->u) {   // no dense coarsest inverse, or nothing fits: kernel by kernel
     if ((rc0 = mg_alloc_field(m, w))) return rc0;
     uniform_faces64<<<nb(m->ncell), MGT, 0, m->stream>>>(S, w->gE64, w->gS64, w->gB64);
@@ -1789,10 +1794,6 @@ static int mg_build(hsb_dev_model *m, MgWork *w) {
       mg_diag<<<nb(L.ncell), MGT, 0, m->stream>>>(dev_level(m, L, l), L.diag);
     }
     HSB_CUDA(cudaGetLastError());
-  }
-  if (!uni) {
-    u_free(w->u);
-    w->u = nullptr;
   }
   // the coarse levels that fuse into one single-CTA kernel: from the first
   // level of at most MG_FUSE_PLANE columns whose levels down to the coarsest

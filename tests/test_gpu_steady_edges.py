@@ -3,7 +3,7 @@ something they cannot solve, or meet a model that has changed."""
 import numpy as np
 import pytest
 
-from hotspot_b200 import FORM_FAST, STEADY_AUTO, STEADY_BICGSTAB
+from hotspot_b200 import FORM_FAST, STEADY_AUTO, STEADY_BICGSTAB, _abi
 from hotspot_b200 import model as hm
 from hotspot_b200 import workloads as W
 from hotspot_b200._abi import HotspotError
@@ -111,7 +111,7 @@ def test_mg_single_level_refinements(workdir, rows, cols, tol):
 def test_mg_out_of_memory_then_again(workdir):
     """A steady solve that runs out of device memory while it sets its workspace
     up (the last of its vectors does not fit) reports that, and the model solves
-    once there is room."""
+    once there is room; nothing stays allocated."""
     import torch
 
     sc = _chip(workdir, 1024, 1024, False)
@@ -152,3 +152,25 @@ def test_mg_out_of_memory_then_again(workdir):
         m.close()
         assert free() > base - vec
     assert raised >= 2
+
+
+@pytest.mark.parametrize("rows,cols", [(4, 8), (32, 32), (256, 128)])
+def test_mg_after_an_operator_without_inverse(workdir, rows, cols):
+    """A model that has solved, then gets conductances of zero throughout (its
+    coarsest operator has no inverse any more): the solve reports that it cannot,
+    and with the conductances back it gives the same bits."""
+    sc = _chip(workdir, rows, cols, False)
+    m = hm.from_scenario(sc)
+    m.set_solver(FORM_FAST)
+    p, s, t = m.power_vector(sc.block_power[0]), m.vector(), m.vector()
+    m.steady(p.copy(), s)
+    inf = np.full(52, np.inf)
+    L = _abi.lib()
+    assert L.hsb_dev_set_layers(L.hsb_grid_device(m.ptr), *[_abi.dptr(inf)] * 5, m.config.ambient, 0.016, 0.016, 0.0) == 0
+    with pytest.raises(HotspotError):
+        m.steady(p.copy(), t)
+    hm.populate_R_model(m, m._flp)
+    hm.populate_C_model(m, m._flp)
+    m.steady(p.copy(), t)
+    assert np.array_equal(s, t)
+    m.close()
