@@ -704,6 +704,17 @@ static void fill_packx(const hsb_dev_model *m, PackX *P) {
   }
 }
 
+// The kernel reads a cell's six resistances at once, also the ones towards
+// neighbours the grid does not have and whose quotients it drops; a grid one
+// cell wide may come without arrays of those, and any array stands in.
+static StencilArgs exact_args(const hsb_dev_model *m) {
+  StencilArgs A = make_args(m, m->L0, m->nr, m->nc);
+  const double **r[6] = {&A.rN, &A.rS, &A.rW, &A.rE, &A.rA, &A.rB};
+  for (const double **p : r)
+    if (!*p) *p = m->pgrid;
+  return A;
+}
+
 static const void *exact_kernel(int v) {
   return v == 0 ? (const void *)rk4_exact_kernel<false, false> : v == 1 ? (const void *)rk4_exact_kernel<false, true>
          : v == 2 ? (const void *)rk4_exact_kernel<true, false> : (const void *)rk4_exact_kernel<true, true>;
@@ -747,7 +758,7 @@ static int exact_prepare(hsb_dev_model *m, XWork **out) {
     HSB_CUDA(h2d_on(w->px, &P, sizeof(P), m->stream));
     if (m->field) {
       if (!w->z) HSB_CUDA(cudaMalloc((void **)&w->z, sizeof(double) * 7 * m->ncell));
-      xfield_recip<<<(unsigned)((m->ncell + 255) / 256), 256, 0, m->stream>>>(make_args(m, m->L0, m->nr, m->nc), w->z);
+      xfield_recip<<<(unsigned)((m->ncell + 255) / 256), 256, 0, m->stream>>>(exact_args(m), w->z);
       HSB_CUDA(cudaGetLastError());
     }
     w->px_version = m->coef_version;
@@ -762,6 +773,9 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   XWork *w = nullptr;
   int rc;
   if (m->vlen >= (1LL << 31) - 1) return set_error(HSB_E_NOMEM, "transient: more than 2^31 cells");   // 17 GB a vector
+  if (m->field && (!m->cap || (m->nr > 1 && !(m->rN && m->rS)) || (m->nc > 1 && !(m->rW && m->rE)) ||
+                   (m->nl > 1 && !(m->rA && m->rB))))
+    return set_error(HSB_E_ARG, "transient: the cells lack resistances or capacitances");
   if ((rc = exact_prepare(m, &w))) return rc;
   const int v = (m->field ? 2 : 0) + (m->uchan_mask ? 1 : 0);
   const void *fn = exact_kernel(v);
@@ -780,7 +794,7 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   while (nt < XTMAX && (m->ncell + nt - 1) / nt + 1 > w->nsm) nt *= 2;
   XArgs G;
   memset(&G, 0, sizeof(G));
-  G.A = make_args(m, m->L0, m->nr, m->nc);
+  G.A = exact_args(m);
   G.F.z = w->z;
   G.px = w->px;
   G.el[0] = m->hsidx; G.el[1] = m->spidx; G.el[2] = m->pcbidx; G.el[3] = m->solderidx; G.el[4] = m->subidx;
