@@ -66,15 +66,20 @@ namespace hsb {
 struct XCtl {                 // the kernel's report
   double t, h, max;
   long long steps, attempts;
-  int yi, ik1, ik1n, ik1p;    // roles of the buffers at the end
+  int yi;                     // which of the two state buffers holds the state at the end
   int status;                 // X_DONE or X_POW (the host decides the attempt)
   int lost;                   // raised by a CTA whose grid barrier did not complete
 };
 enum { X_DONE = 0, X_POW = 1 };
 
-// per-cell coefficients: reciprocals of A.rN, rS, rE, rW, rA, rB and cap, one array after another
+// per-cell coefficients: reciprocals of A.rN, rS, rE, rW, rA, rB and cap, one
+// array (st apart) after another.  Where they did not fit into device memory
+// all of them are one zero (st and mask 0): xdiv's quotients are then out of its
+// range and every cell takes the plain divisions, the same doubles.
 struct XField {
   const double *z;
+  long long st;
+  unsigned mask;
 };
 
 struct PackX;
@@ -86,24 +91,24 @@ struct XArgs {
   int txl;                    // log2 of the tile width
   int cwl;                    // log2 of the package CTA's chunk width
   int tiles, ntj, nti;
-  double *Y[2], *k[3], *X[4], *acc[2], *t1;
+  double *Y[2], *k[2], *t1, *C, *D, *acc;   // see XRole; D null: no speculation
   const double *p;
   unsigned *bar;              // bar, err[2] and ctl are zeroed before the launch
   unsigned long long *err;
   XCtl *ctl;
   double T, t, h;
-  int yi, ik1, ik1n, ik1p;
+  int yi, ik1;
   int have_k1;                // k[ik1] holds k1 of the attempt
 };
 
 struct XWork {
   double *slab;
-  double *v[10];
+  double *v[6];               // k1 and kb, t1, C, acc, D (null where it did not fit)
   unsigned *bar;
   unsigned long long *err;
   XCtl *ctl;
   PackX *px;
-  double *z;                  // reciprocals of the per-cell coefficients (field models)
+  double *z, *zero;           // reciprocals of the per-cell coefficients (field models); a zero
   int px_version;
   int nsm;
   bool ready[4];              // per kernel variant: shared memory limit raised
@@ -149,9 +154,22 @@ struct LayerX {
 // node c; the operation order is that of rk4_core (RCutil.c:469-527)
 enum { XP_K1, XP_1, XP_2, XP_3, XP_4, XP_4S, XP_5, XP_6, XP_7 };
 
+//
+// A vector's place is taken again as soon as its last reader has passed a grid
+// barrier, so eight hold a step (the state's two among them):
+//   yn   the full step's input of pass 2; ytemp from pass 3 on
+//   t1   the half step's input of pass 2; t1 from pass 3 on
+//   C    the full step's input of pass 3; the inputs of passes 5 and 7
+//   D    the half step's input of pass 3; the input of pass 6
+//   kb   the half step's running sum up to pass 3; f(t1) from pass 4 on, k1 of
+//        a retry (which changes places with k1)
+//   k1   k1 up to pass 1; f(ytemp) from pass 4 on, k1 of the next step
+//   acc  the running sum of the full step, then of the second half step
+// D takes the place of k1 where a model is so large that there was no room for
+// it: f(ytemp) then has none, and the next step begins with k1 = f(y).
 struct XRole {
   const double *y;            // base of the stage (y, or t1 in passes 5-7)
-  double *yn, *t1, *k1, *k1n, *k1p, *Xa0, *Xa1, *Xb0, *Xb1, *acca, *accb;
+  double *yn, *t1, *k1, *kb, *C, *D, *acc;
   double h, hb;               // full and half step
 };
 
@@ -161,47 +179,47 @@ struct XOwn {
   double b, c, d;             // stage base; running sums of the one or two cores
 };
 template <int P>
-__device__ __forceinline__ XOwn xown(const XRole &r, int c) {
+__device__ __forceinline__ XOwn xown(const XRole &r, unsigned c) {
   XOwn o{0.0, 0.0, 0.0};
   if (P == XP_1 || P == XP_2 || P == XP_3) o.b = r.y[c];
   if (P >= XP_4) o.b = r.t1[c];
   if (P == XP_1) o.c = r.k1[c];
   if (P == XP_2 || P == XP_3) {
-    o.c = r.acca[c];
-    o.d = r.accb[c];
+    o.c = r.acc[c];
+    o.d = r.kb[c];
   }
-  if (P == XP_5) o.c = r.k1p[c];
-  if (P == XP_6 || P == XP_7) o.c = r.acca[c];
+  if (P == XP_5) o.c = r.kb[c];
+  if (P == XP_6 || P == XP_7) o.c = r.acc[c];
   if (P == XP_7) o.d = r.yn[c];
   return o;
 }
 template <int P>
-__device__ __forceinline__ double xepi(const XRole &r, int c, const XOwn &o, double ka, double kb) {
+__device__ __forceinline__ double xepi(const XRole &r, unsigned c, const XOwn &o, double ka, double kb) {
   if (P == XP_K1) {
     r.k1[c] = ka;
   } else if (P == XP_1) {
-    r.acca[c] = o.c + 2 * ka;
-    r.accb[c] = o.c + 2 * kb;
-    r.Xa0[c] = o.b + r.h / 2.0 * ka;
-    r.Xb0[c] = o.b + r.hb / 2.0 * kb;
+    r.acc[c] = o.c + 2 * ka;
+    r.kb[c] = o.c + 2 * kb;
+    r.yn[c] = o.b + r.h / 2.0 * ka;
+    r.t1[c] = o.b + r.hb / 2.0 * kb;
   } else if (P == XP_2) {
-    r.acca[c] = o.c + 2 * ka;
-    r.accb[c] = o.d + 2 * kb;
-    r.Xa1[c] = o.b + r.h * ka;
-    r.Xb1[c] = o.b + r.hb * kb;
+    r.acc[c] = o.c + 2 * ka;
+    r.kb[c] = o.d + 2 * kb;
+    r.C[c] = o.b + r.h * ka;
+    r.D[c] = o.b + r.hb * kb;
   } else if (P == XP_3) {
     r.yn[c] = o.b + xdiv6(r.h * (o.c + ka));
     r.t1[c] = o.b + xdiv6(r.hb * (o.d + kb));
   } else if (P == XP_4 || P == XP_4S) {
-    r.k1p[c] = ka;
-    if (P == XP_4S) r.k1n[c] = kb;
-    r.Xa0[c] = o.b + r.hb / 2.0 * ka;
+    r.kb[c] = ka;
+    if (P == XP_4S) r.k1[c] = kb;
+    r.C[c] = o.b + r.hb / 2.0 * ka;
   } else if (P == XP_5) {
-    r.acca[c] = o.c + 2 * ka;
-    r.Xa1[c] = o.b + r.hb / 2.0 * ka;
+    r.acc[c] = o.c + 2 * ka;
+    r.D[c] = o.b + r.hb / 2.0 * ka;
   } else if (P == XP_6) {
-    r.acca[c] = o.c + 2 * ka;
-    r.Xa0[c] = o.b + r.hb * ka;
+    r.acc[c] = o.c + 2 * ka;
+    r.C[c] = o.b + r.hb * ka;
   } else {
     const double t2 = o.b + xdiv6(r.hb * (o.c + ka));
     return fabs(o.d - t2);   // RCutil.c:592
@@ -235,7 +253,8 @@ __device__ __noinline__ double xslope_plain(const XShared &sh, const TA ta, cons
 // L2 and not one per neighbour.
 template <bool FIELD, bool ADV, bool TWO>
 struct XCell {
-  int n, i, j, c;
+  int n, i, j;
+  unsigned c;
   double pw, Ta, Tb, xa[6], xb[TWO ? 6 : 1];   // power, own value, N S E W above below
   double y[FIELD ? 7 : 1], z[FIELD ? 7 : 1], am[ADV ? 6 : 1];
   XOwn o;
@@ -243,8 +262,9 @@ struct XCell {
 
 template <bool FIELD, bool ADV, int P, bool TWO, class TA, class TB>
 __device__ __forceinline__ void xload(const XShared &sh, const TA &ta, const TB &tb, XCell<FIELD, ADV, TWO> &C) {
-  const int nr = sh.nr, nc = sh.nc, nl = sh.G.A.nl, plane = nr * nc, c = C.c, i = C.i, j = C.j, n = C.n;
-  const int at[6] = {i > 0 ? c - nc : c, i < nr - 1 ? c + nc : c, j < nc - 1 ? c + 1 : c, j > 0 ? c - 1 : c,
+  const int nr = sh.nr, nc = sh.nc, nl = sh.G.A.nl, i = C.i, j = C.j, n = C.n;
+  const unsigned c = C.c, plane = (unsigned)nr * nc;
+  const unsigned at[6] = {i > 0 ? c - nc : c, i < nr - 1 ? c + nc : c, j < nc - 1 ? c + 1 : c, j > 0 ? c - 1 : c,
                      n > 0 ? c - plane : c, n < nl - 1 ? c + plane : c};
   C.pw = sh.G.p[c];
   C.Ta = ta(c);
@@ -260,7 +280,7 @@ __device__ __forceinline__ void xload(const XShared &sh, const TA &ta, const TB 
 #pragma unroll
     for (int f = 0; f < 7; f++) {
       C.y[f] = R[f][c];
-      C.z[f] = sh.G.F.z[f * A.ncell + c];
+      C.z[f] = sh.G.F.z[f * sh.G.F.st + (c & sh.G.F.mask)];
     }
   }
   if constexpr (ADV) {
@@ -299,7 +319,7 @@ __device__ __forceinline__ void xslope(const XShared &sh, const TA &ta, const TB
   }
   if (L.kind != LK_PLAIN) {
     auto edge = [&](int side, const XDiv &d) {
-      const int node = nl * nr * nc + L.base + side;
+      const unsigned node = (unsigned)nl * nr * nc + L.base + side;
       sa += xdiv(ta(node) - C.Ta, d, bad);
       if (TWO) sb += xdiv(tb(node) - C.Tb, d, bad);
     };
@@ -484,7 +504,8 @@ template <bool FIELD, bool ADV, int P, bool TWO, class TA, class TB>
 __device__ __noinline__ double xpass(XShared &sh, double *buf, const TA ta, const TB tb) {
   const XRole &r = sh.r;
   if (blockIdx.x == gridDim.x - 1) {
-    const int t = threadIdx.x, nx = sh.nx, c = (int)sh.ncell + t;
+    const int t = threadIdx.x, nx = sh.nx;
+    const unsigned c = (unsigned)sh.ncell + t;
     XOwn o{0.0, 0.0, 0.0};
     if (t < nx) o = xown<P>(r, c);
     xpack(sh, buf, ta, tb, TWO ? 2 : 1);
@@ -500,7 +521,7 @@ __device__ __noinline__ double xpass(XShared &sh, double *buf, const TA ta, cons
     C.i = (row - C.n * nti) * th + ty;
     C.j = ((tile - row * ntj) << txl) + tx;
     const bool in = C.i < nr && C.j < nc;
-    C.c = (C.n * nr + C.i) * nc + C.j;   // fewer than 2^31 cells: checked by the host
+    C.c = ((unsigned)C.n * nr + C.i) * nc + C.j;   // fewer than 2^32 cells: checked by the host
     return in;
   };
   for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x - 1) {
@@ -555,7 +576,7 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
   }
   __syncthreads();
   unsigned target = 0;
-  int yi = G.yi, ik1 = G.ik1, ik1n = G.ik1n, ik1p = G.ik1p, slot = 0;
+  int yi = G.yi, slot = 0;
   double t = G.t, h = G.h, mx = 0.0;
   long long steps = 0, attempts = 0;
   int status = X_DONE;
@@ -564,9 +585,8 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
     if (tid == 0) {
       XRole &r = sh.r;
       r.y = G.Y[yi]; r.yn = G.Y[yi ^ 1]; r.t1 = G.t1;
-      r.k1 = G.k[ik1]; r.k1n = G.k[ik1n]; r.k1p = G.k[ik1p];
-      r.Xa0 = G.X[0]; r.Xa1 = G.X[1]; r.Xb0 = G.X[2]; r.Xb1 = G.X[3];
-      r.acca = G.acc[0]; r.accb = G.acc[1];
+      r.k1 = G.k[G.ik1]; r.kb = G.k[G.ik1 ^ 1];
+      r.C = G.C; r.D = G.D ? G.D : r.k1; r.acc = G.acc;
       r.h = h;
       r.hb = h / 2.0;
     }
@@ -578,21 +598,21 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
       grid_barrier(G.bar, target, sh.lost);
     }
     const double rem = G.T - t - h;
-    const bool spec = rem >= MIN_STEP * DELTA;   // another step follows this one
+    const bool spec = G.D && rem >= MIN_STEP * DELTA;   // another step follows this one
     xpass<FIELD, ADV, XP_1, true>(sh, xbuf, XForm{r.y, r.k1, r.h / 2.0}, XForm{r.y, r.k1, r.hb / 2.0});
     grid_barrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_2, true>(sh, xbuf, XVec{r.Xa0}, XVec{r.Xb0});
+    xpass<FIELD, ADV, XP_2, true>(sh, xbuf, XVec{r.yn}, XVec{r.t1});
     grid_barrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_3, true>(sh, xbuf, XVec{r.Xa1}, XVec{r.Xb1});
+    xpass<FIELD, ADV, XP_3, true>(sh, xbuf, XVec{r.C}, XVec{r.D});
     grid_barrier(G.bar, target, sh.lost);
     if (spec) xpass<FIELD, ADV, XP_4S, true>(sh, xbuf, XVec{r.t1}, XVec{r.yn});
     else xpass<FIELD, ADV, XP_4, false>(sh, xbuf, XVec{r.t1}, none);
     grid_barrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_5, false>(sh, xbuf, XVec{r.Xa0}, none);
+    xpass<FIELD, ADV, XP_5, false>(sh, xbuf, XVec{r.C}, none);
     grid_barrier(G.bar, target, sh.lost);
-    xpass<FIELD, ADV, XP_6, false>(sh, xbuf, XVec{r.Xa1}, none);
+    xpass<FIELD, ADV, XP_6, false>(sh, xbuf, XVec{r.D}, none);
     grid_barrier(G.bar, target, sh.lost);
-    double err = xpass<FIELD, ADV, XP_7, false>(sh, xbuf, XVec{r.Xa0}, none);
+    double err = xpass<FIELD, ADV, XP_7, false>(sh, xbuf, XVec{r.C}, none);
     for (int o = 16; o > 0; o >>= 1) err = fmax(err, __shfl_down_sync(0xffffffffu, err, o));
     __syncthreads();
     if ((tid & 31) == 0) sh.wmax[tid >> 5] = err;
@@ -622,17 +642,13 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
     t += h;
     if (!(t < G.T && new_h >= MIN_STEP * DELTA)) break;
     h = new_h;
-    // f(ytemp) is the next step's k1 (computed whenever another step follows)
-    const int o = ik1;
-    ik1 = ik1n;
-    ik1n = o;
-    have = spec;
+    have = spec;   // f(ytemp), the next step's k1, is in k1's place
   }
   if (blockIdx.x == 0 && tid == 0) {
     XCtl &c = *G.ctl;
     c.t = t; c.h = h; c.max = mx;
     c.steps = steps; c.attempts = attempts;
-    c.yi = yi; c.ik1 = ik1; c.ik1n = ik1n; c.ik1p = ik1p;
+    c.yi = yi;
     c.status = status;
   }
   if (sh.lost && tid == 0) G.ctl->lost = 1;
@@ -737,17 +753,22 @@ static int exact_prepare(hsb_dev_model *m, XWork **out) {
   if (!w) {
     w = new XWork();
     const size_t vec = ((size_t)m->vlen + 31) / 32 * 32;
-    cudaError_t e = cudaMalloc((void **)&w->slab, sizeof(double) * vec * 10 + XTAIL + sizeof(PackX));
-    if (e != cudaSuccess) {
-      free_exact(w);
-      return cuda_check(e, "allocating the transient's work vectors");
+    int nv = 6;
+    cudaError_t e;
+    while ((e = cudaMalloc((void **)&w->slab, sizeof(double) * vec * nv + XTAIL + sizeof(PackX) + 8)) != cudaSuccess) {
+      const int rc = cuda_check(e, "allocating the transient's work vectors");
+      if (e != cudaErrorMemoryAllocation || --nv < 5) {
+        free_exact(w);
+        return rc;
+      }
     }
-    for (int k = 0; k < 10; k++) w->v[k] = w->slab + k * vec;
-    unsigned char *tail = (unsigned char *)(w->slab + 10 * vec);
+    for (int k = 0; k < nv; k++) w->v[k] = w->slab + k * vec;
+    unsigned char *tail = (unsigned char *)(w->slab + nv * vec);
     w->bar = (unsigned *)tail;
     w->err = (unsigned long long *)(tail + 128);
     w->ctl = (XCtl *)(tail + 256);
     w->px = (PackX *)(tail + XTAIL);
+    w->zero = (double *)(tail + XTAIL + sizeof(PackX));
     w->px_version = -1;
     m->exact = w;
     m->exact_free = free_exact;
@@ -756,10 +777,20 @@ static int exact_prepare(hsb_dev_model *m, XWork **out) {
     PackX P;
     fill_packx(m, &P);
     HSB_CUDA(h2d_on(w->px, &P, sizeof(P), m->stream));
+    HSB_CUDA(cudaMemsetAsync(w->zero, 0, sizeof(double), m->stream));
     if (m->field) {
-      if (!w->z) HSB_CUDA(cudaMalloc((void **)&w->z, sizeof(double) * 7 * m->ncell));
-      xfield_recip<<<(unsigned)((m->ncell + 255) / 256), 256, 0, m->stream>>>(exact_args(m), w->z);
-      HSB_CUDA(cudaGetLastError());
+      if (!w->z) {
+        const cudaError_t e = cudaMalloc((void **)&w->z, sizeof(double) * 7 * m->ncell);
+        if (e != cudaSuccess) {
+          const int rc = cuda_check(e, "allocating the cells' reciprocals");
+          if (e != cudaErrorMemoryAllocation) return rc;
+          w->z = nullptr;
+        }
+      }
+      if (w->z) {
+        xfield_recip<<<(unsigned)((m->ncell + 255) / 256), 256, 0, m->stream>>>(exact_args(m), w->z);
+        HSB_CUDA(cudaGetLastError());
+      }
     }
     w->px_version = m->coef_version;
   }
@@ -772,7 +803,7 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   if (!(0.0 < time_elapsed && h0 >= MIN_STEP * DELTA)) return HSB_OK;   // the loop's own condition
   XWork *w = nullptr;
   int rc;
-  if (m->vlen >= (1LL << 31) - 1) return set_error(HSB_E_NOMEM, "transient: more than 2^31 cells");   // 17 GB a vector
+  if (m->vlen >= 1LL << 32) return set_error(HSB_E_NOMEM, "transient: more than 2^32 cells");   // 34 GB a vector
   if (m->field && (!m->cap || (m->nr > 1 && !(m->rN && m->rS)) || (m->nc > 1 && !(m->rW && m->rE)) ||
                    (m->nl > 1 && !(m->rA && m->rB))))
     return set_error(HSB_E_ARG, "transient: the cells lack resistances or capacitances");
@@ -795,7 +826,9 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   XArgs G;
   memset(&G, 0, sizeof(G));
   G.A = exact_args(m);
-  G.F.z = w->z;
+  G.F.z = w->z ? w->z : w->zero;
+  G.F.st = w->z ? m->ncell : 0;
+  G.F.mask = w->z ? ~0u : 0u;
   G.px = w->px;
   G.el[0] = m->hsidx; G.el[1] = m->spidx; G.el[2] = m->pcbidx; G.el[3] = m->solderidx; G.el[4] = m->subidx;
   int txl = 0;
@@ -805,15 +838,12 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
   G.ntj = (m->nc + (1 << txl) - 1) >> txl;
   G.nti = (m->nr + (nt >> txl) - 1) / (nt >> txl);
   G.tiles = G.ntj * G.nti * m->nl;
-  for (int k = 0; k < 3; k++) G.k[k] = w->v[k];
-  for (int k = 0; k < 4; k++) G.X[k] = w->v[3 + k];
-  G.acc[0] = w->v[7]; G.acc[1] = w->v[8];
-  G.t1 = w->v[9];
+  G.k[0] = w->v[0]; G.k[1] = w->v[1];
+  G.t1 = w->v[2]; G.C = w->v[3]; G.acc = w->v[4]; G.D = w->v[5];
   G.p = m->pgrid;
   G.bar = w->bar; G.err = w->err; G.ctl = w->ctl;
   G.T = time_elapsed;
   G.t = 0.0; G.h = h0;
-  G.ik1 = 0; G.ik1n = 1; G.ik1p = 2;
   G.Y[0] = m->y; G.Y[1] = m->ytemp;
   const int grid = w->nsm < G.tiles + 1 ? w->nsm : G.tiles + 1;
   for (;;) {
@@ -827,7 +857,7 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
     st->rk4_steps += c.steps;
     st->rk4_attempts += c.attempts;
     st->slope_evals += c.steps + 10 * c.attempts;   // as the reference's loop counts them
-    G.yi = c.yi; G.ik1 = c.ik1; G.ik1n = c.ik1n; G.ik1p = c.ik1p;
+    G.yi = c.yi;
     G.t = c.t;
     bool more = false;
     if (c.lost) return set_error(HSB_E_CUDA, "transient: a grid barrier did not complete in time");
@@ -845,22 +875,17 @@ int rk4_exact_run(hsb_dev_model *m, double time_elapsed, double h0, hsb_stats *s
       more = true;
       if (new_h < h) {
         // retry: its k1 is f(t1) of the rejected attempt (RCutil.c:568)
-        const int o = G.ik1;
-        G.ik1 = G.ik1p;
-        G.ik1p = o;
+        G.ik1 ^= 1;
         G.have_k1 = 1;
         G.h = new_h;
       } else {
         const double rem = time_elapsed - G.t - h;
-        G.have_k1 = rem >= MIN_STEP * DELTA;   // the kernel's own condition for f(ytemp)
+        G.have_k1 = G.D && rem >= MIN_STEP * DELTA;   // the kernel's own condition for f(ytemp)
         new_h = HMIN(new_h, rem);
         G.yi ^= 1;
         G.t += h;
         st->rk4_steps += 1;
         st->slope_evals += 1;
-        const int o = G.ik1;
-        G.ik1 = G.ik1n;
-        G.ik1n = o;
         G.h = new_h;
         more = G.t < time_elapsed && new_h >= MIN_STEP * DELTA;
       }

@@ -1,5 +1,5 @@
 """What the exact replay's transient kernel is given and takes: per-cell arrays
-that a grid has no use for."""
+that a grid has no use for, and device memory."""
 import ctypes as C
 
 import numpy as np
@@ -77,3 +77,43 @@ def test_cells_without_the_arrays_they_do_not_need(workdir, rows, cols):
         assert rc != 0 and b"lack" in L.hsb_dev_last_error()
         L.hsb_dev_destroy(dev)
     m.close()
+
+
+@pytest.mark.parametrize("detailed", [False, True])
+def test_work_vectors_and_short_memory(workdir, detailed):
+    """A step keeps six vectors beside the model's four (and the reciprocals of
+    per-cell coefficients).  Where memory is short it does with five and without
+    the reciprocals, no more than the launch per stage kept, and gives the same
+    bits: two intervals with rejected attempts."""
+    import torch
+
+    sc = W.scenario_chip2d(workdir, seed=8, grid=512, steps=1, n_blocks=4)
+    sc.detailed_3D = detailed
+
+    def free():
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.mem_get_info()[0]
+
+    def run(room):
+        m = hm.from_scenario(sc)
+        before = free()
+        hog = torch.empty(before - room, dtype=torch.uint8, device="cuda") if room else None
+        p, t = m.power_vector(sc.block_power[0]), m.vector(m.config.init_temp)
+        m.compute_temp(p.copy(), t, 1e-5)
+        del hog
+        used = before - free()
+        m.compute_temp(p.copy(), None, 2e-3)
+        st, y = m.stats(), m.grid("trans")
+        m.close()
+        return used, st, y
+
+    vec = 8 * 4 * 512 * 512
+    run(0)                    # loads the kernels
+    used, st, y = run(0)
+    assert st["rk4_attempts"] > st["rk4_steps"]
+    assert used <= (6.5 + 7 * detailed) * vec
+    short, sts, ys = run(int(5.6 * vec))
+    assert short <= 5.6 * vec
+    assert (st["rk4_steps"], st["rk4_attempts"], st["slope_evals"]) == (sts["rk4_steps"], sts["rk4_attempts"], sts["slope_evals"])
+    assert np.array_equal(y, ys)
