@@ -1415,6 +1415,7 @@ static int bc_rhs(hsb_dev_model *m, BcWork *w) {
 static void bc_half_sweep(hsb_dev_model *m, BcWork *w, BcSweep &A, int color, float *eout) {
   A.color = color;
   A.eout = eout;
+  if (color && A.L.nc < 2) return;   // a grid of one column: no planes of this colour
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
   cfg.gridDim = dim3(color ? A.L.nc / 2 : (A.L.nc + 1) / 2);

@@ -174,3 +174,22 @@ def test_mg_after_an_operator_without_inverse(workdir, rows, cols):
     m.steady(p.copy(), t)
     assert np.array_equal(s, t)
     m.close()
+
+
+@pytest.mark.parametrize("rows,cols", [(8, 1), (64, 1), (1, 8), (1, 1)])
+def test_bicgstab_steady_of_a_single_column(workdir, rows, cols):
+    """A grid of one column has no planes of the second colour; the plane solver
+    gives what the multigrid solver gives.  Both stop with corrections of 1e-7 K
+    at most, and contract by more than ten."""
+    sc = _chip(workdir, rows, cols, False)
+    m, g = hm.from_scenario(sc), hm.from_scenario(sc)
+    m.set_solver(FORM_FAST, STEADY_BICGSTAB)
+    g.set_solver(FORM_FAST)
+    p, s, t = m.power_vector(sc.block_power[0]), m.vector(), m.vector()
+    for _ in range(2):
+        m.steady(p.copy(), s)
+    g.steady(p.copy(), t)
+    assert np.max(t) > m.config.ambient + 1.0
+    assert np.max(np.abs(s - t)) < 1e-6
+    m.close()
+    g.close()
