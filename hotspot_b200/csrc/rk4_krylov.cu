@@ -904,7 +904,9 @@ int rk4_krylov_complete(hsb_dev_model *m, FastWork *w, double T, hsb_stats *st, 
   *h_next = 0.0;
   *done = (int)w->h_cnt[7];
   if (w->h_cnt[2] == 1) return set_error(HSB_E_NOCONV, "fast transient: RK4 attempt cap reached");
-  if (w->h_cnt[2] == 2) return set_error(HSB_E_CUDA, "fast transient: a tile copy did not complete in time");
+  if (w->h_cnt[2] == 2)
+    return set_error(HSB_E_CUDA, pair_is_kernel(w->kfn) ? "fast transient: a grid barrier did not complete in time"
+                                                        : "fast transient: a tile copy did not complete in time");
   if (w->h_cnt[2] == 3) {
     *t_done = tout[0];
     *h_next = tout[1];
