@@ -625,7 +625,7 @@ def run_ours(args):
     barrier()
     clk = clocks.stop()
     fast_state = m.grid("trans")
-    head_kernel = m.transient_kernel()
+    head_kernel = m.transient_kernel_name()
     if args.profile:
         print(json.dumps({"profile_case": True, "intervals": K, "device_ms": dev_ms,
                           "kernel_ms": ker_ms, "rk4_steps": steps_total}), flush=True)
@@ -754,10 +754,7 @@ def run_ours(args):
     # the kernel's own events; if the library could not time it, the whole interval
     kernel_timed = ker_ms > 0
     achieved = alg_bytes_launch / (((ker_ms if kernel_timed else dev_ms) / K) / 1e3) / 1e9
-    # the pass-by-pass form keeps grids that fit the SMs' shared memory there
-    passes = "rk4_pair_kernel" if args.grid <= 256 else "rk4_krylov_kernel"
-    kname = {"passes": passes, "blocked": "rk4_tb_kernel"}.get(head_kernel, head_kernel)
-    traffic = profiled_traffic(f"{kname}_stack256.md")
+    traffic = profiled_traffic(f"{head_kernel}_stack256.md")
     line = {
         "metric": METRIC, "value": value, "unit": "cell-steps/s", "n_gpus": ws, "steps": K,
         "warmup": Wm, "ms_per_step": dev_ms_max / K, "higher_is_better": True, "scaling": "weak",
@@ -767,7 +764,7 @@ def run_ours(args):
                 "d2h_bytes_per_step": d2h},
         "steady_solves_per_s": {"fast": steady_fast, "unit": "solves/s",
                                 "fast_final_fp64_residual_W": steady_fast_residual},
-        "roofline": {"bound": "hbm", "kernel": kname, "achieved": achieved, "peak": peak,
+        "roofline": {"bound": "hbm", "kernel": head_kernel, "achieved": achieved, "peak": peak,
                      "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": traffic,
                      "alg_bytes_per_launch": alg_bytes_launch,

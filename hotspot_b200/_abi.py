@@ -232,6 +232,7 @@ _SIGS = {
     "hsb_dev_get_state": (C.c_int, [C.c_void_p, C.c_int, _D]),
     "hsb_dev_workspaces": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
     "hsb_dev_transient_kernel": (C.c_int, [C.c_void_p, C.POINTER(C.c_int)]),
+    "hsb_dev_transient_kernel_name": (C.c_char_p, [C.c_void_p]),
     "hsb_dev_steady_leakage": (C.c_int, [C.c_void_p, _D, _D, _D, _D, C.c_void_p, C.POINTER(C.c_int), C.c_void_p]),
     "hsb_dev_set_tile": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "hsb_dev_set_state": (C.c_int, [C.c_void_p, C.c_int, _D]),

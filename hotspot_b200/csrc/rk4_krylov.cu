@@ -935,3 +935,10 @@ extern "C" int hsb_dev_transient_kernel(const hsb_dev_model *m, int *kind) {
   }
   return HSB_OK;
 }
+
+extern "C" const char *hsb_dev_transient_kernel_name(const hsb_dev_model *m) {
+  const hsb::FastWork *w = m ? (const hsb::FastWork *)m->fast : nullptr;
+  if (!w || !w->kfn) return "";
+  if (w->kfn == hsb::tb_kernel(false) || w->kfn == hsb::tb_kernel(true)) return "rk4_tb_kernel";
+  return hsb::pair_is_kernel(w->kfn) ? "rk4_pair_kernel" : "rk4_krylov_kernel";
+}

@@ -235,6 +235,11 @@ class RCModel:
             raise _abi.HotspotError(lib().hsb_dev_last_error().decode(errors="replace").strip())
         return {0: "", 1: "blocked", 2: "blocked_fp64", 3: "passes"}[k.value]
 
+    def transient_kernel_name(self) -> str:
+        """The same by the kernel's own name: "passes" is rk4_pair_kernel where
+        the SMs can hold the grid, else rk4_krylov_kernel."""
+        return lib().hsb_dev_transient_kernel_name(lib().hsb_grid_device(self.ptr)).decode()
+
     def stats(self) -> dict:
         s = _abi.Stats()
         check(lib().hsb_grid_get_stats(self.ptr, C.byref(s)))

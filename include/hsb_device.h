@@ -309,8 +309,12 @@ int hsb_dev_workspaces(const hsb_dev_model *m, int *mask);
  * fast interval): 0 none yet, or HSB_TK_* */
 #define HSB_TK_BLOCKED      1   /* temporally blocked, FP32 passes */
 #define HSB_TK_BLOCKED_FP64 2   /* temporally blocked, FP64 passes */
-#define HSB_TK_PASSES       3   /* one grid-wide pass per Krylov vector */
+#define HSB_TK_PASSES       3   /* one grid-wide pass per Krylov vector, or two at a time */
 int hsb_dev_transient_kernel(const hsb_dev_model *m, int *kind);
+/* the same by the kernel's own name ("" before the first fast interval);
+ * HSB_TK_PASSES is rk4_pair_kernel where the SMs can hold the grid, else
+ * rk4_krylov_kernel */
+const char *hsb_dev_transient_kernel_name(const hsb_dev_model *m);
 
 /* which: 0 = transient state (last_trans), 1 = steady state (last_steady);
  * n = nl*nr*nc + n_extra doubles */

@@ -271,6 +271,23 @@ def test_paired_passes_shapes(workdir, rows, cols, dt):
         x.close()
 
 
+@pytest.mark.parametrize("rows,cols,kernel", [(4, 8, "rk4_pair_kernel"), (128, 64, "rk4_pair_kernel"),
+                                              (1024, 64, "rk4_pair_kernel"), (1024, 128, "rk4_krylov_kernel")])
+def test_which_pass_kernel_runs(workdir, rows, cols, kernel):
+    """The paired passes take every grid that tiles of 512 columns put on the
+    SMs (75776 columns on 148) and no larger one; a model told to go pass by
+    pass never takes them."""
+    sc = W.scenario_stack3d(workdir, seed=1, grid=16, steps=1, n_blocks=3)
+    sc.config.update(grid_rows=str(rows), grid_cols=str(cols))
+    for form, want in ((FORM_FAST, kernel), (FORM_FAST_PASSES, "rk4_krylov_kernel")):
+        m = hm.from_scenario(sc)
+        m.set_solver(form)
+        assert m.transient_kernel_name() == ""
+        m.compute_temp(m.power_vector(sc.block_power[0]), m.vector(m.config.init_temp), sc.dt)
+        assert m.transient_kernel_name() == want and m.transient_kernel() == "passes"
+        m.close()
+
+
 def _narrow(workdir, by):
     """Scale the x extents of every floorplan in the directory."""
     for f in glob.glob(os.path.join(workdir, "*.flp")):
