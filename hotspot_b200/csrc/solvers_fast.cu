@@ -1591,7 +1591,9 @@ int bicgstab_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   const StencilArgs S = make_args(m, m->L0, m->nr, m->nc);
   const long long n0 = m->vlen;
   const double tol = (o && o->steady_tol > 0) ? o->steady_tol : 1e-7;
-  const int max_ref = (o && o->max_iters > 0) ? o->max_iters : 40;
+  // as in the multigrid solver.  Grids of two orders more rows than columns need
+  // 30 to 50 passes, which differ by a third with the rounding of their sums.
+  const int max_ref = (o && o->max_iters > 0) ? o->max_iters : 60;
   double *T = m->ys;
   double *sc = w->red;
   unsigned long long *maxbits = (unsigned long long *)(w->red + RED_MAXBITS);

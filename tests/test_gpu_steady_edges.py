@@ -193,3 +193,18 @@ def test_bicgstab_steady_of_a_single_column(workdir, rows, cols):
     assert np.max(np.abs(s - t)) < 1e-6
     m.close()
     g.close()
+
+
+def test_bicgstab_steady_of_many_passes(workdir):
+    """A grid of 128 times more rows than columns, among the slowest to converge:
+    solved within the default number of passes.  Bar: the fast form's (0.01 K)."""
+    from oracle.restatement import OracleModel
+
+    sc = W.scenario_chip2d(workdir, seed=3588, grid=16, steps=1, n_blocks=5)
+    sc.config.update(grid_rows="512", grid_cols="4")
+    m, o = hm.from_scenario(sc), OracleModel(sc)
+    m.set_solver(FORM_FAST, STEADY_BICGSTAB)
+    p = m.power_vector(sc.block_power[0])
+    m.steady(p.copy(), m.vector())
+    assert np.max(np.abs(m.grid("steady") - o.steady_direct(p)[0])) <= 0.01
+    m.close()
