@@ -1215,7 +1215,7 @@ static int u_iteration(hsb_dev_model *m, MgWork *w, int it, int n_it) {
   mgu_apply<NL><<<grid(u.L[0]), MGU_T, 0, m->stream>>>(u.L[0], w->d_ps, w->z, w->p, u.p2, u.par, w->q, u.epart,
                                                        u.seg, u.part, sc, tk,
                                                        it == 0);
-  const long long n = w->lv[0].n;
+  const long long n = m->vlen;
   mgu_step<<<(unsigned)((n / 4 + 256) / 256), 256, 0, m->stream>>>(w->e, w->rr, w->p, u.p2, u.par, w->q, sc, n, it == 0);
   return HSB_OK;
 }
@@ -1277,7 +1277,7 @@ static cudaError_t mg_alloc(Tp **p, size_t bytes, cudaStream_t s) {
 
 static int mg_setup(hsb_dev_model *m, MgWork *w) {
   w->coef_version = -1;
-  const int nl = m->nl, nx = m->nx;
+  const int nl = m->nl;
   // levels: halve while both sides are even and >= 4 (keep >= 2x2 columns)
   int nr = m->nr, nc = m->nc;
   while (true) {
@@ -1285,7 +1285,9 @@ static int mg_setup(hsb_dev_model *m, MgWork *w) {
     L.nr = nr; L.nc = nc;
     L.plane = (long long)nr * nc;
     L.ncell = L.plane * nl;
-    L.n = L.ncell + nx;
+    // every slot of the package, also those the model has no node for: the
+    // kernel-by-kernel form writes them as zeros and its coarsest solve reads them
+    L.n = L.ncell + NXP;
     w->lv.push_back(L);
     if (nr < 8 || nc < 8 || (nr & 1) || (nc & 1) || L.plane <= 16) break;
     nr /= 2; nc /= 2;

@@ -208,3 +208,45 @@ def test_bicgstab_steady_of_many_passes(workdir):
     m.steady(p.copy(), m.vector())
     assert np.max(np.abs(m.grid("steady") - o.steady_direct(p)[0])) <= 0.01
     m.close()
+
+
+@pytest.mark.parametrize("detailed", [False, True])
+@pytest.mark.parametrize("rows,cols,chip_layers", [(17, 31, 1), (33, 48, 2), (100, 100, 1), (300, 200, 1), (300, 300, 1),
+                                                   (8, 2, 5), (300, 200, 8)])
+def test_mg_kernel_by_kernel_vectors(workdir, rows, cols, chip_layers, detailed):
+    """The kernel-by-kernel form, on grids where a level's vector and its package
+    slots end at the end of the memory they are given (the coarsest level too
+    large for a dense inverse, or per-cell coefficients): every solve of a model
+    gives the same bits, with the layers' resistances and with the same ones cell
+    by cell, and is a solution by its FP64 residual (33x48 is a single level that
+    the smoother alone does not solve within the default passes: the bits of where
+    it gives up)."""
+    import ctypes as C
+
+    from test_gpu_exact_workspace import _device_model
+
+    m = hm.from_scenario(W.scenario_random_chip(workdir, np.random.default_rng(2), "x", side=32, chip_layers=chip_layers,
+                                                steps=1))
+    L, layer, nl = _abi.lib(), [m.ptr.contents.layers[n] for n in range(m.n_layers)], m.n_layers
+    per_cell = lambda v: np.repeat(np.asarray(v, dtype=np.float64), rows * cols)
+    ns, ew = per_cell([l.rx for l in layer]), per_cell([l.ry for l in layer])
+    cells = [ns, ns, ew, ew, per_cell([0.0] + [l.rz for l in layer[:-1]]), per_cell([l.rz for l in layer]),
+             per_cell([l.c for l in layer])]
+    p, out = np.zeros(13), np.zeros(13)
+    p[0] = 20.0
+    states = []
+    for a in ((cells,) if detailed or rows * cols == 16 else (None, cells)):   # (8x2 per layer runs in the cluster)
+        dev = _device_model(m, rows, cols, a)
+        for _ in range(2):
+            st, opts = _abi.Stats(), _abi.SolverOpts(FORM_FAST, STEADY_AUTO, 0.0, 0)
+            rc = L.hsb_dev_steady(dev, _abi.dptr(p), _abi.dptr(out), C.byref(opts), C.byref(st))
+            assert rc == 0 or (rows == 33 and b"did not converge" in L.hsb_dev_last_error()), L.hsb_dev_last_error()
+            y = np.zeros(nl * rows * cols + 12)
+            assert L.hsb_dev_get_state(dev, 1, _abi.dptr(y)) == 0
+            assert rc or st.residual < 1e-5
+            assert np.min(y) > m.config.ambient
+            states.append(y)
+        L.hsb_dev_destroy(dev)
+    for y in states[1:]:
+        assert np.array_equal(y, states[0])
+    m.close()
