@@ -1024,11 +1024,6 @@ __global__ void __launch_bounds__(MGT) add_correction(double *__restrict__ T, co
   }
 }
 
-__global__ void copy_f(const float *__restrict__ a, float *__restrict__ b, long long n) {
-  long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < n) b[k] = a[k];
-}
-
 // right-hand side in FP64: P + ambient conductances * ambient
 __global__ void build_rhs64(const hsb::StencilArgs S, const double *__restrict__ pgrid,
                             const double *__restrict__ gAmb, const double *__restrict__ gamb64,
@@ -1125,7 +1120,6 @@ static void free_mg(void *p);
 // ---------------------------------------------------------------------------
 // per-layer models: mg_uniform.cuh's kernels
 // ---------------------------------------------------------------------------
-#define MGU_TICKETS 16
 struct MgUniform {
   int nlev, small;             // levels small .. nlev - 1 run in mgu_small
   ULev L[24];

@@ -132,7 +132,7 @@ __device__ __forceinline__ double xdiv6(double x) {
   return bad ? x / 6.0 : q;
 }
 
-// the package node equations of pack_slope (temperature_grid.c:2857-3093),
+// the package node equations of slope_fn_pack (temperature_grid.c:2857-3093),
 // one row per node: dv = (edge sum / edgeR + (t0 + t1 + t2)) / C, with
 // t_q = (x_nb - x) / R; every resistance is the double the reference divides
 // by.  A node with fewer terms has itself as the neighbour of the others,
@@ -655,7 +655,7 @@ __global__ void __launch_bounds__(XTMAX, 1) rk4_exact_kernel(const __grid_consta
 }
 
 // the package rows of the model (the same sums of resistances and
-// capacitances as pack_slope, in its order)
+// capacitances as slope_fn_pack, in its order)
 static void fill_packx(const hsb_dev_model *m, PackX *P) {
   memset(P, 0, sizeof(*P));
   const package_RC_t &pk = m->h_pk;

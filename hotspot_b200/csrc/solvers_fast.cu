@@ -987,8 +987,8 @@ __device__ __forceinline__ float bc_row(const BcLevelDev &L, const float *__rest
 // ---------------------------------------------------------------------------
 // BiCGStab vector kernels: FP32 data, FP64 reductions in a fixed order
 // ---------------------------------------------------------------------------
-// scalars: sc[0] rho, [1] rho_old, [2] alpha, [3] omega, [4..9] dot results
-enum { SC_RHO = 0, SC_RHO_OLD, SC_ALPHA, SC_OMEGA, SC_D0, SC_D1, SC_D2, SC_D3, SC_NE, SC_MAX };
+// scalars: rho, rho_old, alpha, omega, the correction's norm
+enum { SC_RHO = 0, SC_RHO_OLD, SC_ALPHA, SC_OMEGA, SC_NE, SC_MAX };
 #define BC_DOT_BLOCKS 592
 // layout of BcWork::red: scalars, max-norm bits, dot partials, edge conductances
 #define RED_MAXBITS SC_MAX

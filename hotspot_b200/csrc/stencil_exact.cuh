@@ -129,156 +129,8 @@ __device__ __forceinline__ double slope_cell_exact(const StencilArgs &A, const T
   return (p[c] + psum) / (FIELD ? A.cap[c] : Ln.cap);
 }
 
-// sequential edge sums sum_k (T_edge_k - x) in the reference's loop order
-template <class TV>
-__device__ __forceinline__ double edge_sum_exact(const StencilArgs &A, const TV &tv,
-                                                  int layer, int which, double x) {
-  // which: 0 = row 0, 1 = row nr-1, 2 = col 0, 3 = col nc-1
-  double s = 0.0;
-  const long long base = (long long)layer * A.plane;
-  if (which < 2) {
-    const long long r = base + (which == 0 ? 0 : (long long)(A.nr - 1) * A.nc);
-    for (int j = 0; j < A.nc; j++) s += (tv(r + j) - x);
-  } else {
-    const long long cc = base + (which == 2 ? 0 : A.nc - 1);
-    for (int i = 0; i < A.nr; i++) s += (tv(cc + (long long)i * A.nc) - x);
-  }
-  return s;
-}
-
-// Package-node slopes (slope_fn_pack, temperature_grid.c:2857-3093).
-// x: the n_extra node temperatures; es: edge sums in the order
-// SINK_C_N,S,W,E, SP_N,S,W,E, [PCB_C_N,S,W,E, SOLDER_N,S,W,E, SUB_N,S,W,E];
-// eNS/eEW of the sink/spreader/... layers are the edge resistances.
-__device__ __forceinline__ void pack_slope_exact(const StencilArgs &A, const double *x,
-                                                 const double *es, double *dv,
-                                                 int spidx, int hsidx, int subidx,
-                                                 int solderidx, int pcbidx) {
-  const package_RC_t *pk = A.pk;
-  const double amb = A.ambient;
-  const LayerCoef &Ls = A.L[spidx], &Lh = A.L[hsidx];
-  double psum;
-  /* sink outer north/south */
-  psum = (amb - x[HSB_SINK_N]) / (pk->r_hs_per + pk->r_amb_per) +
-         (x[HSB_SINK_C_N] - x[HSB_SINK_N]) / (pk->r_hs2_y + pk->r_hs);
-  dv[HSB_SINK_N] = psum / (pk->c_hs_per + pk->c_amb_per);
-  psum = (amb - x[HSB_SINK_S]) / (pk->r_hs_per + pk->r_amb_per) +
-         (x[HSB_SINK_C_S] - x[HSB_SINK_S]) / (pk->r_hs2_y + pk->r_hs);
-  dv[HSB_SINK_S] = psum / (pk->c_hs_per + pk->c_amb_per);
-  /* sink outer west/east */
-  psum = (amb - x[HSB_SINK_W]) / (pk->r_hs_per + pk->r_amb_per) +
-         (x[HSB_SINK_C_W] - x[HSB_SINK_W]) / (pk->r_hs2_x + pk->r_hs);
-  dv[HSB_SINK_W] = psum / (pk->c_hs_per + pk->c_amb_per);
-  psum = (amb - x[HSB_SINK_E]) / (pk->r_hs_per + pk->r_amb_per) +
-         (x[HSB_SINK_C_E] - x[HSB_SINK_E]) / (pk->r_hs2_x + pk->r_hs);
-  dv[HSB_SINK_E] = psum / (pk->c_hs_per + pk->c_amb_per);
-  /* sink inner north/south */
-  psum = es[0] / Lh.edgeNS;
-  psum += (amb - x[HSB_SINK_C_N]) / (pk->r_hs_c_per_y + pk->r_amb_c_per_y) +
-          (x[HSB_SP_N] - x[HSB_SINK_C_N]) / pk->r_sp_per_y +
-          (x[HSB_SINK_N] - x[HSB_SINK_C_N]) / (pk->r_hs2_y + pk->r_hs);
-  dv[HSB_SINK_C_N] = psum / (pk->c_hs_c_per_y + pk->c_amb_c_per_y);
-  psum = es[1] / Lh.edgeNS;
-  psum += (amb - x[HSB_SINK_C_S]) / (pk->r_hs_c_per_y + pk->r_amb_c_per_y) +
-          (x[HSB_SP_S] - x[HSB_SINK_C_S]) / pk->r_sp_per_y +
-          (x[HSB_SINK_S] - x[HSB_SINK_C_S]) / (pk->r_hs2_y + pk->r_hs);
-  dv[HSB_SINK_C_S] = psum / (pk->c_hs_c_per_y + pk->c_amb_c_per_y);
-  /* sink inner west/east */
-  psum = es[2] / Lh.edgeEW;
-  psum += (amb - x[HSB_SINK_C_W]) / (pk->r_hs_c_per_x + pk->r_amb_c_per_x) +
-          (x[HSB_SP_W] - x[HSB_SINK_C_W]) / pk->r_sp_per_x +
-          (x[HSB_SINK_W] - x[HSB_SINK_C_W]) / (pk->r_hs2_x + pk->r_hs);
-  dv[HSB_SINK_C_W] = psum / (pk->c_hs_c_per_x + pk->c_amb_c_per_x);
-  psum = es[3] / Lh.edgeEW;
-  psum += (amb - x[HSB_SINK_C_E]) / (pk->r_hs_c_per_x + pk->r_amb_c_per_x) +
-          (x[HSB_SP_E] - x[HSB_SINK_C_E]) / pk->r_sp_per_x +
-          (x[HSB_SINK_E] - x[HSB_SINK_C_E]) / (pk->r_hs2_x + pk->r_hs);
-  dv[HSB_SINK_C_E] = psum / (pk->c_hs_c_per_x + pk->c_amb_c_per_x);
-  /* spreader north/south */
-  psum = es[4] / Ls.edgeNS;
-  psum += (x[HSB_SINK_C_N] - x[HSB_SP_N]) / pk->r_sp_per_y;
-  dv[HSB_SP_N] = psum / pk->c_sp_per_y;
-  psum = es[5] / Ls.edgeNS;
-  psum += (x[HSB_SINK_C_S] - x[HSB_SP_S]) / pk->r_sp_per_y;
-  dv[HSB_SP_S] = psum / pk->c_sp_per_y;
-  /* spreader west/east */
-  psum = es[6] / Ls.edgeEW;
-  psum += (x[HSB_SINK_C_W] - x[HSB_SP_W]) / pk->r_sp_per_x;
-  dv[HSB_SP_W] = psum / pk->c_sp_per_x;
-  psum = es[7] / Ls.edgeEW;
-  psum += (x[HSB_SINK_C_E] - x[HSB_SP_E]) / pk->r_sp_per_x;
-  dv[HSB_SP_E] = psum / pk->c_sp_per_x;
-
-  if (A.secondary) {
-    const LayerCoef &Lp = A.L[pcbidx], &Lq = A.L[solderidx], &Lb = A.L[subidx];
-    /* PCB outer north/south */
-    psum = (amb - x[HSB_PCB_N]) / (pk->r_amb_sec_per) +
-           (x[HSB_PCB_C_N] - x[HSB_PCB_N]) / (pk->r_pcb2_y + pk->r_pcb);
-    dv[HSB_PCB_N] = psum / (pk->c_pcb_per + pk->c_amb_sec_per);
-    psum = (amb - x[HSB_PCB_S]) / (pk->r_amb_sec_per) +
-           (x[HSB_PCB_C_S] - x[HSB_PCB_S]) / (pk->r_pcb2_y + pk->r_pcb);
-    dv[HSB_PCB_S] = psum / (pk->c_pcb_per + pk->c_amb_sec_per);
-    /* PCB outer west/east */
-    psum = (amb - x[HSB_PCB_W]) / (pk->r_amb_sec_per) +
-           (x[HSB_PCB_C_W] - x[HSB_PCB_W]) / (pk->r_pcb2_x + pk->r_pcb);
-    dv[HSB_PCB_W] = psum / (pk->c_pcb_per + pk->c_amb_sec_per);
-    psum = (amb - x[HSB_PCB_E]) / (pk->r_amb_sec_per) +
-           (x[HSB_PCB_C_E] - x[HSB_PCB_E]) / (pk->r_pcb2_x + pk->r_pcb);
-    dv[HSB_PCB_E] = psum / (pk->c_pcb_per + pk->c_amb_sec_per);
-    /* PCB inner north/south */
-    psum = es[8] / Lp.edgeNS;
-    psum += (amb - x[HSB_PCB_C_N]) / (pk->r_amb_sec_c_per_y) +
-            (x[HSB_SOLDER_N] - x[HSB_PCB_C_N]) / pk->r_pcb_c_per_y +
-            (x[HSB_PCB_N] - x[HSB_PCB_C_N]) / (pk->r_pcb2_y + pk->r_pcb);
-    dv[HSB_PCB_C_N] = psum / (pk->c_pcb_c_per_y + pk->c_amb_sec_c_per_y);
-    psum = es[9] / Lp.edgeNS;
-    psum += (amb - x[HSB_PCB_C_S]) / (pk->r_amb_sec_c_per_y) +
-            (x[HSB_SOLDER_S] - x[HSB_PCB_C_S]) / pk->r_pcb_c_per_y +
-            (x[HSB_PCB_S] - x[HSB_PCB_C_S]) / (pk->r_pcb2_y + pk->r_pcb);
-    dv[HSB_PCB_C_S] = psum / (pk->c_pcb_c_per_y + pk->c_amb_sec_c_per_y);
-    /* PCB inner west/east */
-    psum = es[10] / Lp.edgeEW;
-    psum += (amb - x[HSB_PCB_C_W]) / (pk->r_amb_sec_c_per_x) +
-            (x[HSB_SOLDER_W] - x[HSB_PCB_C_W]) / pk->r_pcb_c_per_x +
-            (x[HSB_PCB_W] - x[HSB_PCB_C_W]) / (pk->r_pcb2_x + pk->r_pcb);
-    dv[HSB_PCB_C_W] = psum / (pk->c_pcb_c_per_x + pk->c_amb_sec_c_per_x);
-    psum = es[11] / Lp.edgeEW;
-    psum += (amb - x[HSB_PCB_C_E]) / (pk->r_amb_sec_c_per_x) +
-            (x[HSB_SOLDER_E] - x[HSB_PCB_C_E]) / pk->r_pcb_c_per_x +
-            (x[HSB_PCB_E] - x[HSB_PCB_C_E]) / (pk->r_pcb2_x + pk->r_pcb);
-    dv[HSB_PCB_C_E] = psum / (pk->c_pcb_c_per_x + pk->c_amb_sec_c_per_x);
-    /* solder north/south */
-    psum = es[12] / Lq.edgeNS;
-    psum += (x[HSB_PCB_C_N] - x[HSB_SOLDER_N]) / pk->r_pcb_c_per_y;
-    dv[HSB_SOLDER_N] = psum / pk->c_solder_per_y;
-    psum = es[13] / Lq.edgeNS;
-    psum += (x[HSB_PCB_C_S] - x[HSB_SOLDER_S]) / pk->r_pcb_c_per_y;
-    dv[HSB_SOLDER_S] = psum / pk->c_solder_per_y;
-    /* solder west/east */
-    psum = es[14] / Lq.edgeEW;
-    psum += (x[HSB_PCB_C_W] - x[HSB_SOLDER_W]) / pk->r_pcb_c_per_x;
-    dv[HSB_SOLDER_W] = psum / pk->c_solder_per_x;
-    psum = es[15] / Lq.edgeEW;
-    psum += (x[HSB_PCB_C_E] - x[HSB_SOLDER_E]) / pk->r_pcb_c_per_x;
-    dv[HSB_SOLDER_E] = psum / pk->c_solder_per_x;
-    /* substrate north/south */
-    psum = es[16] / Lb.edgeNS;
-    psum += (x[HSB_SOLDER_N] - x[HSB_SUB_N]) / pk->r_solder_per_y;
-    dv[HSB_SUB_N] = psum / pk->c_sub_per_y;
-    psum = es[17] / Lb.edgeNS;
-    psum += (x[HSB_SOLDER_S] - x[HSB_SUB_S]) / pk->r_solder_per_y;
-    dv[HSB_SUB_S] = psum / pk->c_sub_per_y;
-    /* substrate west/east */
-    psum = es[18] / Lb.edgeEW;
-    psum += (x[HSB_SOLDER_W] - x[HSB_SUB_W]) / pk->r_solder_per_x;
-    dv[HSB_SUB_W] = psum / pk->c_sub_per_x;
-    psum = es[19] / Lb.edgeEW;
-    psum += (x[HSB_SOLDER_E] - x[HSB_SUB_E]) / pk->r_solder_per_x;
-    dv[HSB_SUB_E] = psum / pk->c_sub_per_x;
-  }
-}
-
-// (layer, edge) of each package edge sum, in pack_slope_exact's es[] order
+// (layer, edge) of each package edge sum, in the order SINK_C_N,S,W,E, SP_N,S,W,E,
+// [PCB_C_N,S,W,E, SOLDER_N,S,W,E, SUB_N,S,W,E]
 __device__ __forceinline__ void edge_desc(int e, int spidx, int hsidx, int subidx, int solderidx,
                                           int pcbidx, int *layer, int *which, int *node) {
   // node groups: SINK_C_* (4), SP_* (0), PCB_C_* (20), SOLDER_* (16), SUB_* (12);
