@@ -2014,7 +2014,8 @@ int mg_steady(hsb_dev_model *m, const hsb_solver_opts *o, hsb_stats *st) {
   // model runs each pass iteration by iteration and offers to yield between
   // them, so that it holds the device for one iteration at most after a
   // priority request arrives; otherwise one graph per pass
-  const bool pieces = m->yield_fn && m->ncell >= MG_YIELD_SPLIT_CELLS && inner > 1;
+  // (a pass that is one launch of mgu_small has no pieces)
+  const bool pieces = m->yield_fn && m->ncell >= MG_YIELD_SPLIT_CELLS && inner > 1 && !(w->u && w->u->pcg);
   const int inner_next = MG_INNER_NEXT < inner ? MG_INNER_NEXT : inner;
   if (!pieces && (!w->pass_exec || w->pass_T != T || w->pass_version != m->coef_version)) {
     if ((rc = capture([&]() {
