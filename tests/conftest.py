@@ -7,6 +7,12 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 if ROOT not in sys.path:
     sys.path.insert(0, ROOT)
 
+# a reference directory without the sources counts as none (test modules skip on
+# a path that does not exist)
+_ref = os.environ.get("HOTSPOT_REFERENCE_SRC", "/root/reference")
+if not os.path.isfile(os.path.join(_ref, "temperature_grid.c")):
+    os.environ["HOTSPOT_REFERENCE_SRC"] = os.path.join(_ref, "no-sources")
+
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA GPU (B200, sm_100a)")
