@@ -488,8 +488,8 @@ def leg_microchannel(args):
             "roofline": {"bound": "hbm", "kernel": "BiCGStab iteration (bc_*)", "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind, "traffic": None,
                          "note": "104 B per cell per iteration algorithmic (unpreconditioned BiCGStab's streams); "
-                                 "the V-cycle preconditioner's plane solves are sequential chains, so the "
-                                 "iteration is latency-bound, not HBM-bound"},
+                                 "the V-cycle preconditioner is a chain of half sweeps, each waiting for the one "
+                                 "before, so the iteration is latency-bound, not HBM-bound"},
             "cpu_baseline": {"kind": "port", "what": "FP64 sparse LU (scipy splu) of the restated system, 1 thread",
                              "sample": "128x128 model", "s_per_solve": out["128x128"]["cpu_direct_s"]}}
 
@@ -721,14 +721,13 @@ def run_ours(args):
                            "steady_solves_per_s": 1e3 / rp["steady_ms"],
                            "speedup_fast_vs_plain_transient": value / (rp["rate"] * ws),
                            "speedup_fast_vs_plain_steady": steady_fast * rp["steady_ms"] / 1e3,
-                           "what": "the FP64 replay of the reference's RK4 stage by stage (10 stencil kernels per "
-                                   "attempt, host step control with the reference's pow); steady: the replay of its "
-                                   "nested-iteration Gauss-Seidel, stopping where the reference stops"},
+                           "what": "the FP64 replay of the reference's RK4 in its operation order (one cooperative "
+                                   "launch per interval, step sizes with the C library's pow); steady: the replay of "
+                                   "its nested-iteration Gauss-Seidel, stopping where the reference stops"},
             "fp64_blocked": {"cell_steps_per_s": fb["rate"], "gpu_launches": fb["launches"],
                              "speedup_fast_vs_fp64_blocked_transient": value / (fb["rate"] * ws),
                              "max_dT_K_vs_replay": float(np.max(np.abs(fb["state"] - rp["state"]))),
-                             "what": "the temporally blocked Krylov-form kernel with every stencil pass in FP64: "
-                                     "the fastest all-FP64 transient here"},
+                             "what": "the temporally blocked Krylov-form kernel with every stencil pass in FP64"},
             "fast_blocked": {"cell_steps_per_s": tb["rate"], "gpu_launches": tb["launches"],
                              "max_dT_K_vs_replay": float(np.max(np.abs(tb["state"] - rp["state"]))),
                              "what": "the fast form's arithmetic on the temporally blocked kernel (the fast form's "

@@ -26,11 +26,13 @@
 // An iteration at 256x256 is 6 launches where kernel by kernel it was 42, most
 // of them a few microseconds of launch and drain around little work.  Steady
 // states on B200, before and after: 64x64x4 1879 -> 729 us, 256x256x6 3413 ->
-// 1578 us, 1024x1024x5 11047 -> 4642 us.  What is left: mgu_small is bound by
-// its cluster barriers (about 1000 cycles each; 70 us an iteration from 128x128
-// down); the tiled kernels at 1024x1024 (apply 50 us, post 49, down 28, pre 20,
-// step 16) run at up to a quarter of the copy rate.  The residual and correction kernels of mg_steady.cu
-// were bound by one atomic per warp on a single word; they take one per CTA.
+// 1578 us, 1024x1024x5 11047 -> 4642 us.  What is left: mgu_small, 70 us an
+// iteration from 128x128 down, of which 23 cluster barriers of about 1000
+// cycles are 12 us (at 64x64 18 of them, 9 of 29 us) and the rest a chain of
+// dependent phases, some on one SM; the tiled kernels at 1024x1024 (apply 48 us,
+// post 49, down 28, pre 21, step 16) run at up to a quarter of the copy rate.
+// The residual and correction kernels of mg_steady.cu were bound by one atomic
+// per warp on a single word; they take one per CTA.
 #pragma once
 #include <cooperative_groups.h>
 

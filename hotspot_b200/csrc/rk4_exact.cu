@@ -35,8 +35,8 @@
 //
 // Measured on one B200, an interval of four steps through compute_temp, one
 // launch per stage with a host round trip per attempt against this kernel:
-// 64x64x4 632 -> 175 us, 256x256x6 1440 -> 378 us, a 128x128x4 microchannel
-// stack (14 attempts, 8 of them decided on the host) 2260 -> 770 us.  A grid
+// 64x64x4 632 -> 175 us, 256x256x6 1440 -> 374 us, a 128x128x4 microchannel
+// stack (14 attempts, 8 of them decided on the host) 2420 -> 840 us.  A grid
 // barrier is 2.1 thousand cycles of a pass; at 64x64x4 the package CTA's pass
 // is 4.3 to 6 thousand (an FP64 add is 18 cycles, so a 64-cell edge 1.2), at
 // 256x256x6 the cells' is 13.5 for one stage input and 19 for two.
