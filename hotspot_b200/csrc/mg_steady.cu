@@ -972,11 +972,13 @@ __global__ void dot_one(const float *__restrict__ a, const float *__restrict__ b
   }
 }
 
-// a step length of the conjugate gradients.  A residual that is zero to begin
-// with (no power and everything at ambient) has (r, z) = (p, q) = 0: no step.
-// Anything else that does not divide reaches the correction, whose norm then
-// reports it.
-__device__ __forceinline__ float mg_ratio(double a, double b) { return a == 0.0 ? 0.f : (float)(a / b); }
+// a step length of the conjugate gradients, a = (r, z).  No step where the
+// residual is zero (no power and everything at ambient) or so small that what
+// the iteration makes of it leaves FP32's range: an exact coarsest solve takes
+// seven digits off it per iteration, and at the end (p, q) is zero for a residual
+// that is not.  (1e-60: entries of 1e-31 W and 1e-29 K.)  Anything else that does
+// not divide reaches the correction, whose norm then reports it.
+__device__ __forceinline__ float mg_ratio(double a, double b) { return fabs(a) < 1e-60 ? 0.f : (float)(a / b); }
 
 // x += alpha p; r -= alpha q   with alpha = rz / pq  (sc[2] rz, sc[1] pq)
 __global__ void pcg_update_xr(float *__restrict__ x, float *__restrict__ r, const float *__restrict__ p,

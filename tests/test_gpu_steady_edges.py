@@ -250,3 +250,33 @@ def test_mg_kernel_by_kernel_vectors(workdir, rows, cols, chip_layers, detailed)
     for y in states[1:]:
         assert np.array_equal(y, states[0])
     m.close()
+
+
+@pytest.mark.parametrize("detailed", [False, True])
+@pytest.mark.parametrize("rows,cols,chip_layers", [(1, 1, 1), (2, 2, 1), (4, 4, 1), (4, 8, 1), (2, 2, 4), (32, 32, 4)])
+def test_mg_steady_of_next_to_no_power(workdir, rows, cols, chip_layers, detailed):
+    """Residuals that the iteration brings to the end of FP32's range: powers of
+    1e-20 W and less heat by less than a temperature's last place, so everything
+    is at ambient to the bit."""
+    import ctypes as C
+
+    from test_gpu_exact_workspace import _device_model
+
+    m = hm.from_scenario(W.scenario_random_chip(workdir, np.random.default_rng(32), "x", side=32, chip_layers=chip_layers,
+                                                steps=1))
+    L, layer, nl = _abi.lib(), [m.ptr.contents.layers[n] for n in range(m.n_layers)], m.n_layers
+    per_cell = lambda v: np.repeat(np.asarray(v, dtype=np.float64), rows * cols)
+    ns, ew = per_cell([l.rx for l in layer]), per_cell([l.ry for l in layer])
+    cells = [ns, ns, ew, ew, per_cell([0.0] + [l.rz for l in layer[:-1]]), per_cell([l.rz for l in layer]),
+             per_cell([l.c for l in layer])]
+    dev = _device_model(m, rows, cols, cells if detailed else None)
+    p, out, y = np.zeros(13), np.zeros(13), np.zeros(nl * rows * cols + 12)
+    for power in (1e-20, 1e-25, 1e-30, 1e-35, 1e-38, 1e-44, 1e-300):
+        p[0] = power
+        st, opts = _abi.Stats(), _abi.SolverOpts(FORM_FAST, STEADY_AUTO, 0.0, 0)
+        rc = L.hsb_dev_steady(dev, _abi.dptr(p), _abi.dptr(out), C.byref(opts), C.byref(st))
+        assert rc == 0, (power, L.hsb_dev_last_error())
+        assert L.hsb_dev_get_state(dev, 1, _abi.dptr(y)) == 0
+        assert np.array_equal(y, np.full(y.size, m.config.ambient)), power
+    L.hsb_dev_destroy(dev)
+    m.close()
